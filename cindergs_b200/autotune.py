@@ -4,10 +4,10 @@ launch shapes.
 Three parameters are tuned per viewport: the screen tile shape of Stages 3
 and 4 (the reference's 16 x 16 pixels, 8 x 8 or 32 x 16: larger tiles give
 fewer tile entries to bin and sort but more candidate splats per pixel in
-the compositor), and how the tile entries are sorted -- the digit width of
-the radix passes (balanced digits, or 4..8 bits) and the method (radix
-passes or the one-pass tile transpose, where the frame has at most 16,384
-tiles). The sort choices produce the same lists bit for bit; the tile shape
+the compositor), and how the tile lists are made -- the method (screen-block
+lists, radix passes over the tile entries, or the one-pass tile transpose,
+where the frame has at most 16,384 tiles) and the digit width of the radix
+passes (balanced digits, or 4..8 bits). The sort choices produce the same lists bit for bit; the tile shape
 changes a pixel only where the tile test's rounding admits a splat whose
 alpha is below the 1/255 cut there anyway. For each distinct viewport of a
 set of views, one representative view is rendered with every candidate and
@@ -36,6 +36,7 @@ def candidates(width: int, height: int, tile_shapes=TILE_SHAPES):
     for ts in tile_shapes:
         tw, th = _abi.TILE_SHAPES[ts]
         tiles = ((width + tw - 1) // tw) * ((height + th - 1) // th)
+        out.append((ts, 0, _abi.SORT_AUTO))
         out += [(ts, rb, _abi.SORT_RADIX) for rb in DIGIT_WIDTHS]
         if tiles <= 16384:
             out.append((ts, 0, _abi.SORT_TRANSPOSE))

@@ -30,6 +30,7 @@ UNITS = [
     ("stage1_mvc.cu", ["-fmad=false"]),
     ("stage2_project.cu", ["-fmad=false"]),
     ("stage3_bin.cu", []),  # explicit __fmul_rn/__fadd_rn where the keys depend on rounding
+    ("stage3_lists.cu", ["-fmad=false"]),  # explicit too
     ("sh_rotate.cu", ["-fmad=false"]),
     ("springs.cu", ["-fmad=false"]),
     ("radix_sort.cu", []),
@@ -40,7 +41,7 @@ UNITS = [
     ("pipeline.cu", []),
     ("noalloc.cu", []),
 ]
-HEADERS = ["common.cuh", "detmath.h", "kernels.h", "field.h"]
+HEADERS = ["common.cuh", "detmath.h", "kernels.h", "field.h", "tile_test.cuh"]
 
 
 def _nvcc() -> str:

@@ -33,7 +33,7 @@ struct FrameCounters {
   uint32_t status;       // kStatus* bits
   uint32_t fetched;      // splat records the compositor gathered
   uint32_t tile_ctr[16]; // dynamic tile counters for chained-scan kernels
-  uint32_t pad;
+  uint32_t pairs;        // Stage 3 (splat, screen block) pairs
   unsigned long long stage_ctr;  // binning: staged entries so far (64 bits: never wraps)
 };
 // Largest tile-entry capacity of a frame (32-bit entry indices; a multiple
@@ -46,7 +46,7 @@ constexpr uint32_t kMaxEntryCap = 0xFFFF0000u;
 struct __align__(16) SplatRec {
   float4 geo;   // mu_x, mu_y, conic a, conic b
   float4 cc;    // conic c, alpha_2d, t_z, extents (u32 bits: ext_x | ext_y << 16; 0 = culled)
-  float4 rgb;   // r, g, b, unused
+  float4 rgb;   // r, g, b, the tile test's limit on the quadratic form (2 ln(255 alpha) + 1e-4)
 };
 static_assert(sizeof(SplatRec) == 48, "SplatRec must be 48 bytes");
 

@@ -216,6 +216,10 @@ struct ProjectArgs {
   int key64;
   uint32_t depth_base_bits;   // near-plane exponent bits (32-bit keys)
   uint32_t depth_bits;        // depth bits in a 32-bit key
+  // screen-block lists: the blocks each splat's tile box touches (list_box),
+  // or null
+  uint32_t* boxes;            // [max_n]
+  uint32_t tiles_x, tiles_y, tile_w_log2, tile_h_log2, blocks_x;
 };
 cudaError_t launch_project(const ProjectArgs& a, cudaStream_t s);
 
@@ -305,6 +309,80 @@ constexpr uint32_t kTransposeGroupTiles = 2048;  // screen tiles per group (2^11
 cudaError_t launch_chunk_counts(const TransposeArgs& a, cudaStream_t s);
 cudaError_t launch_column_scan(const TransposeArgs& a, cudaStream_t s);
 cudaError_t launch_chunk_place(const TransposeArgs& a, cudaStream_t s);
+
+// ---- Stage 3, screen-block lists (stage3_lists.cu) -----------------------------
+// A screen block is 8x4 screen tiles. Splats in depth order are paired with
+// the blocks their tile boxes touch, the pairs are sorted by block, and every
+// block's pairs are turned into its 32 tiles' lists.
+constexpr uint32_t kListBlockW = 3, kListBlockH = 2;  // log2 of a block's tiles
+constexpr uint32_t kListMaxBlocks = 16384;  // block counters in shared memory, 14-bit block ids
+constexpr uint32_t kListSlots = 1024;       // slots of one pairing tile
+constexpr uint32_t kListSmallPairs = 1u << 18;  // up to here a chunk is one group of 32 pairs
+constexpr uint32_t kListGroups = 4;         // groups of 32 pairs per chunk beyond
+constexpr uint32_t kListSegChunks = 64;     // chunks of one placing segment
+// The screen blocks a splat's tile box touches: first block | width << 14 |
+// height << 23, 0 when the splat has no entries (a box spans at most 1024 + 1
+// + 1024 pixels: 34 x 66 blocks of 8x8-pixel tiles).
+__host__ __device__ inline uint32_t list_box(uint32_t first, uint32_t w, uint32_t h) {
+  return first | (w << 14) | (h << 23);
+}
+// Control words of a frame's lists (zeroed with the frame's scratch).
+struct ListPlan {
+  uint32_t sort_n;        // pairs to sort (0 when they exceed the buffers)
+  uint32_t chunks;        // chunks of all blocks
+  uint32_t groups;        // groups of 32 pairs per chunk
+  uint32_t segs;          // placing segments of all blocks
+  uint32_t done;          // pairing thread blocks that have finished
+  uint32_t slot_ctr;      // pairing tiles taken
+  uint32_t seg_ctr;       // placing segments taken
+  uint32_t pad;
+};
+struct ListArgs {
+  const SplatRec* recs;
+  const uint32_t* order_ids;    // slot -> splat (depth order)
+  const uint32_t* boxes;        // [max_n] list_box of each splat (Stage 2)
+  const uint32_t* split_count;  // null when no splitting
+  uint32_t n_rest, max_n;
+  uint32_t width, height, tiles_x, tiles_y, tile_w_log2, tile_h_log2;
+  uint32_t blocks_x, num_blocks;
+  FrameCounters* fc;
+  ListPlan* plan;
+  unsigned long long* lookback; // [ceil(max_n / kListSlots)] zeroed
+  uint32_t* block_count;        // [num_blocks] pairs per block, zeroed
+  uint32_t* block_start;        // [num_blocks + 1] first pair of each block
+  uint32_t* chunk_first;        // [num_blocks + 1] first chunk of each block
+  uint32_t* seg_first;          // [num_blocks + 1] first placing segment of each block
+  uint32_t* hist;               // pair sort's digit counts [passes][1 << radix_bits]
+  uint32_t radix_bits, passes;
+  uint32_t* pair_blocks;        // [pair_cap] block of each pair, slot order
+  uint32_t* pair_ids;           // [pair_cap] splat of each pair, slot order
+  uint32_t pair_cap;
+  const uint32_t* sorted_pairs; // [pair_cap] splats sorted by (block, slot)
+  uint32_t* masks;              // [chunks * groups][32] ballots of 32 pairs per tile
+  uint32_t* chunk_base;         // [chunks][32] entries per tile -> exclusive over the block's chunks
+  unsigned long long* seg_look; // [segs][32] placing look-back words
+  uint32_t* tile_base;          // [num_blocks][32] first entry of each tile
+  uint32_t* ranges;             // [tiles] (start, end), (0, 0) when empty
+  uint32_t* ids;                // [entry_cap] splat indices, tile by tile
+  uint32_t entry_cap;
+};
+// Chunks, ballot groups and placing segments of a frame of at most pair_cap pairs.
+inline uint32_t list_chunk_cap(uint32_t pair_cap, uint32_t blocks) {
+  const uint32_t all = pair_cap / 32 + 1, most = kListSmallPairs / 32;
+  const uint32_t large = pair_cap / (32 * kListGroups) + 1;
+  const uint32_t small = most < all ? most : all;
+  return (small > large ? small : large) + blocks;
+}
+inline uint32_t list_group_cap(uint32_t pair_cap, uint32_t blocks) {
+  return pair_cap / 32 + 1 + kListGroups * blocks;
+}
+inline uint32_t list_seg_cap(uint32_t pair_cap, uint32_t blocks) {
+  return list_chunk_cap(pair_cap, blocks) / kListSegChunks + 1 + blocks;
+}
+cudaError_t launch_list_pairs(const ListArgs& a, cudaStream_t s);
+cudaError_t launch_list_count(const ListArgs& a, cudaStream_t s);
+cudaError_t launch_list_place(const ListArgs& a, cudaStream_t s);
+cudaError_t launch_list_write(const ListArgs& a, cudaStream_t s);
 
 // Per-tile [start, end) from sorted words: tile = word >> shift, over
 // min(*n_ptr, capacity) words. ranges zeroed.

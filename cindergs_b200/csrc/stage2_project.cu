@@ -17,6 +17,7 @@
 #include <cuda_fp16.h>
 
 #include "kernels.h"
+#include "tile_test.cuh"
 
 namespace cgs {
 namespace {
@@ -127,7 +128,8 @@ __global__ void __launch_bounds__(kProjectMaxThreads, 2) k_project(const Project
     const float ty = w10 * px + w11 * py + w12 * pz + w13;
     const float tz = w20 * px + w21 * py + w22 * pz + w23;
     uint32_t ext_packed = 0;
-    float mu_x = 0, mu_y = 0, ca = 0, cb = 0, cc = 0, alpha_2d = 0;
+    uint32_t box = 0;
+    float mu_x = 0, mu_y = 0, ca = 0, cb = 0, cc = 0, alpha_2d = 0, q_lim = 0;
     const float op = p4.w;
     if (tz > near_p && !(op < a.min_opacity)) {
       const float4 ca4 = a.cova[idx];
@@ -206,6 +208,17 @@ __global__ void __launch_bounds__(kProjectMaxThreads, 2) k_project(const Project
                 cc = sp_xx * inv_det;
                 ext_packed = ((uint32_t)ext_x & 0xFFFFu) | (((uint32_t)ext_y & 0xFFFFu) << 16);
                 visible = true;
+                q_lim = q_max + 1e-4f;
+                if (a.boxes) {
+                  const int32_t mx = (int32_t)a.tiles_x - 1, my = (int32_t)a.tiles_y - 1;
+                  const float itw = __uint_as_float((127u - a.tile_w_log2) << 23);
+                  const float ith = __uint_as_float((127u - a.tile_h_log2) << 23);
+                  const uint32_t x0 = tile_coord(mu_x - ext_x, mx, itw) >> kListBlockW;
+                  const uint32_t x1 = tile_coord(mu_x + ext_x, mx, itw) >> kListBlockW;
+                  const uint32_t y0 = tile_coord(mu_y - ext_y, my, ith) >> kListBlockH;
+                  const uint32_t y1 = tile_coord(mu_y + ext_y, my, ith) >> kListBlockH;
+                  box = list_box(y0 * a.blocks_x + x0, x1 - x0 + 1u, y1 - y0 + 1u);
+                }
               }
             }
           }
@@ -245,7 +258,7 @@ __global__ void __launch_bounds__(kProjectMaxThreads, 2) k_project(const Project
       const float3 rgb = eval_sh(sh.c, dx, dy, dz, deg);
       rec->geo = make_float4(mu_x, mu_y, ca, cb);
       rec->cc = make_float4(cc, alpha_2d, tz, __uint_as_float(ext_packed));
-      rec->rgb = make_float4(rgb.x, rgb.y, rgb.z, 0.0f);
+      rec->rgb = make_float4(rgb.x, rgb.y, rgb.z, q_lim);
     } else {
       rec->cc = make_float4(0.0f, 0.0f, tz, 0.0f);
     }
@@ -266,6 +279,7 @@ __global__ void __launch_bounds__(kProjectMaxThreads, 2) k_project(const Project
       }
       a.depth_keys[idx] = dk;
       a.depth_ids[idx] = idx;
+      if (a.boxes) a.boxes[idx] = box;
     }
   }
   if (idx == 0) a.fc->active = active < a.max_n ? active : a.max_n;

@@ -75,7 +75,7 @@ typedef struct cgs_frame_params {
   int32_t profile_stages;       /* 1: time each stage with CUDA events */
   int32_t force_stage3;         /* 1: never reuse the cached Stage 3 lists */
   int32_t write_f32;            /* 1: also write an unquantised RGBA f32 frame */
-  int32_t radix_bits;           /* entry-sort digit width: 0 = balanced digits of at most
+  int32_t radix_bits;           /* radix entry sort's digit width: 0 = balanced digits of at most
                                    8 bits over the tile bits (13 bits -> 7 + 6), else 4..8 */
   int32_t entry_sort;           /* CGS_SORT_*: how the tile entries are sorted by tile */
   int32_t tile_shape;           /* CGS_TILE_*: screen tile of Stages 3 and 4 */
@@ -93,7 +93,9 @@ typedef struct cgs_frame_params {
 #define CGS_TILE_32X16 2
 
 /* Entry sort methods (the result is the same, bit for bit). */
-#define CGS_SORT_AUTO 0       /* radix passes */
+#define CGS_SORT_AUTO 0       /* screen-block lists: (splat, 8x4-tile block) pairs sorted by
+                                 block, each block's tiles listed by ballots; radix passes
+                                 where a viewport has more than 16,384 blocks */
 #define CGS_SORT_RADIX 1      /* LSD radix passes over the tile bits */
 #define CGS_SORT_TRANSPOSE 2  /* one-pass tile transpose (32-bit keys and at most 16,384
                                  tiles; otherwise radix passes) */
@@ -425,9 +427,11 @@ int cgs_framebuffer_device(cgs_ctx* ctx, void** d_rgba8, uint32_t* row_pitch_px)
 #define CGS_K_TET_TRANSFORMS 1
 #define CGS_K_DEFORM 2
 #define CGS_K_PROJECT 3
-#define CGS_K_BIN 4            /* count + chained scan + key emission, one launch */
-#define CGS_K_ENTRY_SORT 5     /* stable sort of the tile entries by tile: the one-pass
-                                  tile transpose, or radix passes for many tiles */
+#define CGS_K_BIN 4            /* screen-block pairs + tile tests, or (entry sorts) count +
+                                  chained scan + key emission in one launch */
+#define CGS_K_ENTRY_SORT 5     /* pair sort + places + entries of the screen-block lists, or a
+                                  stable sort of the tile entries by tile: radix passes, or the
+                                  one-pass tile transpose */
 #define CGS_K_TILE_RANGES 6    /* (the tile transpose writes the ranges itself) */
 #define CGS_K_COMPOSITE 7
 #define CGS_K_SPLAT_SORT 8     /* depth-key histogram + radix passes over the splats */

@@ -233,11 +233,11 @@ struct cgs_ctx {
   int s3_order_src = 0;    // buffer holding the latest Stage 3's splat order
   bool s3_transpose = false;  // the latest Stage 3 sorted by the tile transpose
   DevBuf cmat;             // tile transpose: [tiles][chunks] counts / first entries
-  // screen-block lists: (block, splat) pairs, their sort's look-back pair, the
-  // groups' hit ballots and the chunks' first entries
-  DevBuf pair_blocks[2], pair_ids[2], pair_lb[2], list_masks, list_base, list_look, list_boxes;
-  uint32_t pair_cap = 0;        // pairs those buffers are wanted for
-  uint32_t pair_lb_tiles = 0;   // tiles the pair sort's look-back buffers cover
+  // screen-block lists: one allocation laid out by ListLayout for list_pairs
+  // pairs and list_blocks blocks, and Stage 2's boxes
+  DevBuf lists, list_boxes;
+  uint32_t list_pairs = 0, list_blocks = 0;
+  uint32_t pair_cap = 0;        // pairs the buffers are wanted for
   int pair_parity = 0;
   bool s3_lists = false;        // the latest Stage 3 went through the lists
   uint32_t entry_cap = 0;       // capacity of the key/id buffers (entries)
@@ -423,27 +423,48 @@ int ensure_entry_buffers(cgs_ctx* ctx, uint32_t cap, bool key64, uint32_t radix_
   return CGS_OK;
 }
 
-// Buffers of the screen-block lists for `cap` entries and `pairs` pairs.
+// Places of the screen-block lists' buffers in their one allocation (a new
+// context's first frame waits for every allocation it makes).
+struct ListLayout {
+  size_t blocks[2], ids[2], lb[2], lb_bytes, masks, base, look, bytes;
+  ListLayout(uint32_t pairs, uint32_t nblocks) {
+    size_t at = 0;
+    auto take = [&](size_t n) {
+      const size_t p = at;
+      at = (at + n + 255) & ~(size_t)255;
+      return p;
+    };
+    // look-back words of the pair sort: 64 bits beyond 2^30 pairs, as for entries
+    lb_bytes = (size_t)sort_tiles(pairs) * 256 * (pairs > (1u << 30) ? 8 : 4);
+    for (int k = 0; k < 2; ++k) lb[k] = take(lb_bytes);
+    for (int k = 0; k < 2; ++k) {
+      blocks[k] = take((size_t)pairs * 4);
+      ids[k] = take((size_t)pairs * 4);
+    }
+    masks = take((size_t)list_group_cap(pairs, nblocks) * 128);
+    base = take((size_t)list_chunk_cap(pairs, nblocks) * 128);
+    look = take((size_t)list_seg_cap(pairs, nblocks) * 256);
+    bytes = at;
+  }
+};
+
+// Buffers of the screen-block lists for `cap` entries and `pairs` pairs
+// (Stage 2's boxes have their own: a re-run after an overflow reads them
+// again). The layout is fixed between changes of the sizes; the
+// pair sort's look-back buffers are cleared with each (its passes clear the
+// one they do not use over the whole grid).
 int ensure_list_buffers(cgs_ctx* ctx, uint32_t cap, uint32_t pairs, uint32_t blocks) {
   CGS_TRY(ctx->ensure(ctx->ids[0], (size_t)std::max(cap, 1u) * 4, "tile lists"));
-  for (int k = 0; k < 2; ++k) {
-    CGS_TRY(ctx->ensure(ctx->pair_blocks[k], (size_t)pairs * 4, "pair blocks"));
-    CGS_TRY(ctx->ensure(ctx->pair_ids[k], (size_t)pairs * 4, "pair splats"));
-  }
-  CGS_TRY(ctx->ensure(ctx->list_masks, (size_t)list_group_cap(pairs, blocks) * 128, "list ballots"));
-  CGS_TRY(ctx->ensure(ctx->list_base, (size_t)list_chunk_cap(pairs, blocks) * 128, "list bases"));
-  CGS_TRY(ctx->ensure(ctx->list_look, (size_t)list_seg_cap(pairs, blocks) * 256, "list look-back"));
-  const uint32_t tiles = sort_tiles(pairs);
-  if (tiles != ctx->pair_lb_tiles || !ctx->pair_lb[0].p) {
-    // 64-bit words beyond 2^30 pairs, as for the entries
-    const size_t bytes = (size_t)tiles * 256 * (pairs > (1u << 30) ? 8 : 4);
-    for (int k = 0; k < 2; ++k) {
-      CGS_TRY(ctx->ensure(ctx->pair_lb[k], bytes, "pair sort look-back"));
-      CGS_CUDA(cudaMemsetAsync(ctx->pair_lb[k].p, 0, bytes, ctx->stream), "clear look-back");
-    }
-    ctx->pair_lb_tiles = tiles;
-    ctx->pair_parity = 0;
-  }
+  if (pairs == ctx->list_pairs && blocks <= ctx->list_blocks && ctx->lists.p) return CGS_OK;
+  blocks = std::max(blocks, ctx->list_blocks);
+  const ListLayout L(pairs, blocks);
+  CGS_TRY(ctx->ensure(ctx->lists, L.bytes, "screen-block lists"));
+  ++ctx->alloc_epoch;  // a captured graph holds the old places
+  for (int k = 0; k < 2; ++k)
+    CGS_CUDA(cudaMemsetAsync(ctx->lists.as<char>() + L.lb[k], 0, L.lb_bytes, ctx->stream), "clear look-back");
+  ctx->list_pairs = pairs;
+  ctx->list_blocks = blocks;
+  ctx->pair_parity = 0;
   return CGS_OK;
 }
 
@@ -502,7 +523,6 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   a.tile_h_log2 = d.tile_lh;
   a.blocks_x = d.blocks_x;
   a.num_blocks = d.num_blocks;
-  a.boxes = ctx->list_boxes.as<uint32_t>();
   a.fc = fc;
   a.plan = (ListPlan*)(sc + L.plan);
   a.lookback = (unsigned long long*)(sc + L.llb);
@@ -511,18 +531,21 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   a.chunk_first = (uint32_t*)(sc + L.lchunk);
   a.seg_first = (uint32_t*)(sc + L.lseg);
   a.tile_base = (uint32_t*)(sc + L.ltile);
-  a.seg_look = ctx->list_look.as<unsigned long long>();
   a.hist = (uint32_t*)(sc + L.hist);
   // balanced digits over the block bits (255 blocks at 1080p: one pass of 8)
   const uint32_t bits = std::max(1u, d.num_blocks <= 1 ? 1u : 32u - (uint32_t)__builtin_clz(d.num_blocks - 1));
   *passes = (bits + 7) / 8;
   a.passes = *passes;
   a.radix_bits = std::max(4u, (bits + *passes - 1) / *passes);
-  a.pair_blocks = ctx->pair_blocks[0].as<uint32_t>();
-  a.pair_ids = ctx->pair_ids[0].as<uint32_t>();
-  a.pair_cap = ctx->pair_cap;
-  a.masks = ctx->list_masks.as<uint32_t>();
-  a.chunk_base = ctx->list_base.as<uint32_t>();
+  const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+  char* lp = ctx->lists.as<char>();
+  a.boxes = ctx->list_boxes.as<uint32_t>();
+  a.seg_look = (unsigned long long*)(lp + B.look);
+  a.pair_blocks = (uint32_t*)(lp + B.blocks[0]);
+  a.pair_ids = (uint32_t*)(lp + B.ids[0]);
+  a.pair_cap = ctx->list_pairs;
+  a.masks = (uint32_t*)(lp + B.masks);
+  a.chunk_base = (uint32_t*)(lp + B.base);
   a.ranges = ctx->ranges.as<uint32_t>();
   a.ids = ctx->ids[0].as<uint32_t>();
   a.entry_cap = ctx->entry_cap;
@@ -531,17 +554,17 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   ctx->kend();
   SortArgs so{};
   for (int k = 0; k < 2; ++k) {
-    so.keys[k] = ctx->pair_blocks[k].as<uint32_t>();
-    so.vals[k] = ctx->pair_ids[k].as<uint32_t>();
-    so.status2[k] = ctx->pair_lb[k].p;
+    so.keys[k] = (uint32_t*)(lp + B.blocks[k]);
+    so.vals[k] = (uint32_t*)(lp + B.ids[k]);
+    so.status2[k] = lp + B.lb[k];
   }
   so.n_ptr = &a.plan->sort_n;
-  so.capacity = ctx->pair_cap;
+  so.capacity = a.pair_cap;
   so.num_bits = bits;
   so.radix_bits = a.radix_bits;
   so.hist = a.hist;
   so.parity = &ctx->pair_parity;
-  so.wide_lookback = ctx->pair_cap > (1u << 30);
+  so.wide_lookback = a.pair_cap > (1u << 30);
   so.lb_stride = 256;
   so.tile_ctr = (uint32_t*)(sc + L.rtiles);
   so.status_word = &fc->status;
@@ -550,7 +573,7 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   ctx->kbegin(CGS_K_ENTRY_SORT);
   CGS_CUDA(run_radix_sort(so, &src, s), "pair sort");
   ctx->kend();
-  a.sorted_pairs = ctx->pair_ids[src].as<uint32_t>();
+  a.sorted_pairs = (const uint32_t*)(lp + B.ids[src]);
   ctx->kbegin(CGS_K_BIN);
   CGS_CUDA(launch_list_count(a, s), "list count launch");
   ctx->kend();
@@ -1141,10 +1164,8 @@ int cgs_ctx_device_bytes(const cgs_ctx* ctx, uint64_t* out) {
                           &ctx->def_cova, &ctx->def_covb, &ctx->split_meta, &ctx->persist,
                           &ctx->recs, &ctx->offsets, &ctx->scratch, &ctx->ranges, &ctx->keys[0],
                           &ctx->keys[1], &ctx->ids[0], &ctx->ids[1], &ctx->depths[0],
-                          &ctx->depths[1], &ctx->radix_lb[0], &ctx->radix_lb[1], &ctx->pair_blocks[0],
-                          &ctx->pair_blocks[1], &ctx->pair_ids[0], &ctx->pair_ids[1],
-                          &ctx->pair_lb[0], &ctx->pair_lb[1], &ctx->list_masks,
-                          &ctx->list_base, &ctx->list_look, &ctx->list_boxes, &ctx->fb_rgba8,
+                          &ctx->depths[1], &ctx->radix_lb[0], &ctx->radix_lb[1], &ctx->lists,
+                          &ctx->list_boxes, &ctx->fb_rgba8,
                           &ctx->fb_f32, &ctx->prim[0], &ctx->prim[1], &ctx->prim[2],
                           &ctx->prim[3]};
   uint64_t t = 0;
@@ -2517,8 +2538,10 @@ int capture_views(cgs_ctx* ctx, uint32_t nv, const cgs_camera* cams, const cgs_c
     if (ctx->radix_lb[k].p) e = cudaMemsetAsync(ctx->radix_lb[k].p, 0, ctx->radix_lb[k].cap, s);
     if (e == cudaSuccess && ctx->splat_lb[k].p)
       e = cudaMemsetAsync(ctx->splat_lb[k].p, 0, ctx->splat_lb[k].cap, s);
-    if (e == cudaSuccess && ctx->pair_lb[k].p)
-      e = cudaMemsetAsync(ctx->pair_lb[k].p, 0, ctx->pair_lb[k].cap, s);
+    if (e == cudaSuccess && ctx->lists.p) {
+      const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+      e = cudaMemsetAsync(ctx->lists.as<char>() + B.lb[k], 0, B.lb_bytes, s);
+    }
   }
   ctx->radix_parity = 0;
   ctx->splat_parity = 0;
@@ -2538,7 +2561,10 @@ int capture_views(cgs_ctx* ctx, uint32_t nv, const cgs_camera* cams, const cgs_c
   for (int k = 0; k < 2; ++k) {
     if (ctx->radix_lb[k].p) cudaMemsetAsync(ctx->radix_lb[k].p, 0, ctx->radix_lb[k].cap, s);
     if (ctx->splat_lb[k].p) cudaMemsetAsync(ctx->splat_lb[k].p, 0, ctx->splat_lb[k].cap, s);
-    if (ctx->pair_lb[k].p) cudaMemsetAsync(ctx->pair_lb[k].p, 0, ctx->pair_lb[k].cap, s);
+    if (ctx->lists.p) {
+      const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+      cudaMemsetAsync(ctx->lists.as<char>() + B.lb[k], 0, B.lb_bytes, s);
+    }
   }
   ctx->views_radix_parity = ctx->radix_parity;
   ctx->views_splat_parity = ctx->splat_parity;

@@ -220,88 +220,124 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) {
   return r;
 }
 
+// n / d in both halves, correctly rounded to binary32, from y = RN(1 / d):
+// Markstein's division (IBM J. Res. Dev. 34(1), 1990). One step makes q
+// faithful; from a faithful q and a correctly rounded reciprocal the second
+// gives the correctly rounded quotient, as long as nothing under- or
+// overflows (3 x 10^9 operand pairs equal n / d). The sign of a zero is lost.
+__device__ __forceinline__ f2 div2(f2 n, f2 neg_d, f2 y) {
+  const f2 q = mul2(n, y);
+  const f2 q1 = fma2(fma2(neg_d, q, n), y, q);
+  return fma2(fma2(neg_d, q1, n), y, q1);
+}
+__device__ __noinline__ f2 div2_ieee(f2 n, f2 neg_d) {
+  float a, b, c, d;
+  unpack2(n, a, b);
+  unpack2(neg_d, c, d);
+  return pack2(__fdiv_rn(a, -c), __fdiv_rn(b, -d));
+}
+
 // The tests of 32 pairs of a block against its 32 tiles, one pair per lane
 // (ellipse_intersects_tile_gpu, binning.rs:37-96, term for term). Per lane the
-// four rows' terms stay in registers and the eight columns are walked; a tile
-// takes two clamps, a compare pair and half of 11 packed products and sums,
-// then one ballot. A tile outside the lane's own tile box fails: its row's
-// limit is NaN, its column's predicate false. Bound by instruction issue
+// four rows' terms stay in registers and the eight columns are walked two at a
+// time; a tile takes two clamps, a compare pair and half of 11 packed products
+// and sums, then one ballot. A tile outside the lane's own tile box fails: its
+// row's limit is NaN, its column's predicate false. Bound by instruction issue
 // (clamps and compares run at half the products' rate).
 __global__ void __launch_bounds__(kListThreads, 3) k_list_count(const ListArgs a, float neg_zero) {
   __shared__ __align__(16) uint32_t s_mask[kListWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunks = a.plan->chunks, groups = a.plan->groups;
   const uint32_t active = min(a.n_rest + (a.split_count ? *a.split_count : 0u), a.max_n);
-  const uint32_t wm1 = a.width - 1u, hm1 = a.height - 1u;
+  const float x_last = pixel_center(a.width - 1u), y_last = pixel_center(a.height - 1u);
   const uint32_t lw = a.tile_w_log2, lh = a.tile_h_log2;
+  const float tw = (float)(1u << lw), th = (float)(1u << lh);
   uint32_t* sm = s_mask[warp];
   const f2 nz = pack2(neg_zero, neg_zero);
   for (uint32_t c = blockIdx.x * kListWarps + warp; c < chunks; c += gridDim.x * kListWarps) {
     const uint32_t b = block_of(a.chunk_first, a.num_blocks, c);
     const uint32_t tx0 = (b % a.blocks_x) << kListBlockW, ty0 = (b / a.blocks_x) << kListBlockH;
     const uint32_t i0 = a.block_start[b] + (c - a.chunk_first[b]) * 32u * groups;
-    const uint32_t end = a.block_start[b + 1];
+    const uint32_t end = min(a.block_start[b + 1], a.pair_cap);
+    // pixel centres are half-integers below 2^22: these sums are exact
+    const float px0 = pixel_center(tx0 << lw), py0 = pixel_center(ty0 << lh);
     uint32_t cnt = 0;
+    uint32_t sid = i0 + lane < end ? a.sorted_pairs[i0 + lane] : kInvalid;
     for (uint32_t j = 0; j < groups && i0 + 32u * j < end; ++j) {
-      const uint32_t i = i0 + 32u * j + lane;
-      const uint32_t sid = i < end && i < a.pair_cap ? a.sorted_pairs[i] : kInvalid;
       const SplatBox bx = load_box(a, sid, active);
       const float lim = bx.valid ? a.recs[sid].rgb.w : 0.0f;
+      const uint32_t nxt = i0 + 32u * (j + 1) + lane;
+      sid = j + 1 < groups && nxt < end ? a.sorted_pairs[nxt] : kInvalid;
       const float nan = __int_as_float(0x7FC00000);
       const float ca_ = fmaxf(bx.ca, 1e-12f), cc_ = fmaxf(bx.cc, 1e-12f);
       const float cb2 = __fmul_rn(2.0f, bx.cb);
       const float ya = __frcp_rn(ca_), yc = __frcp_rn(cc_);
-      const bool okb = fabsf(bx.cb) < 0x1p40f;
-      const bool oka = okb && ca_ <= 0x1p20f, okc = okb && cc_ <= 0x1p20f;
-      float y0[4], y1[4], rz[4], rl[4];
-      f2 rw[2], yn[2];
-      {
-        float w_[4], n_[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const uint32_t ty = ty0 + k, ys = ty << lh;
-          y0[k] = __fsub_rn(pixel_center(ys), bx.mu_y);
-          y1[k] = __fsub_rn(pixel_center(min(ys + ((1u << lh) - 1u), hm1)), bx.mu_y);
-          n_[k] = clampf(0.0f, y0[k], y1[k]);
-          rz[k] = div_rcp32(__fmul_rn(-bx.cb, n_[k]), ca_, ya, oka);
-          w_[k] = __fmul_rn(__fmul_rn(bx.cc, n_[k]), n_[k]);
-          rl[k] = bx.valid && ty >= bx.y0 && ty <= bx.y1 ? lim : nan;
-        }
-        rw[0] = pack2(w_[0], w_[1]);
-        rw[1] = pack2(w_[2], w_[3]);
-        yn[0] = pack2(n_[0], n_[1]);
-        yn[1] = pack2(n_[2], n_[3]);
-      }
+      // a nonzero distance to a pixel centre is at least 2^-25 and below 2^24,
+      // so with these bounds no quotient or residue leaves the normal range
+      const bool ok = (bx.cb == 0.0f || fabsf(bx.cb) >= 0x1p-30f) && fabsf(bx.cb) < 0x1p40f &&
+                      ca_ <= 0x1p20f && cc_ <= 0x1p20f;
+      const bool fast = __all_sync(0xffffffffu, ok || !bx.valid);
       const f2 ca2 = pack2(bx.ca, bx.ca), cc2 = pack2(bx.cc, bx.cc), cb22 = pack2(cb2, cb2);
-#pragma unroll 2
-      for (uint32_t k = 0; k < 8; ++k) {
-        const uint32_t tx = tx0 + k, xs = tx << lw;
-        const bool in = tx >= bx.x0 && tx <= bx.x1;
-        uint32_t m[4] = {0u, 0u, 0u, 0u};
-        if (__any_sync(0xffffffffu, in && bx.valid)) {
-          const float x0 = __fsub_rn(pixel_center(xs), bx.mu_x);
-          const float x1 = __fsub_rn(pixel_center(min(xs + ((1u << lw) - 1u), wm1)), bx.mu_x);
-          const float xn = clampf(0.0f, x0, x1);
-          const float cz = div_rcp32(__fmul_rn(-bx.cb, xn), cc_, yc, okc);
-          const float cw = __fmul_rn(__fmul_rn(bx.ca, xn), xn);
-          const float cp = __fmul_rn(cb2, xn);
-          const f2 cw2 = pack2(cw, cw), cp2 = pack2(cp, cp);
+      const f2 nb2 = pack2(-bx.cb, -bx.cb);
+      float y0[4], y1[4], rz[4], rl[4];
+      f2 yn[4], rw[4];
+      {
+        const f2 nmu = pack2(-bx.mu_y, -bx.mu_y), nd = pack2(-ca_, -ca_), y2 = pack2(ya, ya);
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const f2 y = pack2(clampf(cz, y0[2 * h], y1[2 * h]), clampf(cz, y0[2 * h + 1], y1[2 * h + 1]));
-            const f2 q1 = add2(add2(cw2, fma2(cp2, y, nz)), fma2(mul2(cc2, y), y, nz));
-            const f2 x = pack2(clampf(rz[2 * h], x0, x1), clampf(rz[2 * h + 1], x0, x1));
-            const f2 q2 =
-                add2(add2(fma2(mul2(ca2, x), x, nz), fma2(mul2(cb22, x), yn[h], nz)), rw[h]);
-            float q1a, q1b, q2a, q2b;
-            unpack2(q1, q1a, q1b);
-            unpack2(q2, q2a, q2b);
-            // fminf(q1, q2) <= limit: either is (a NaN never is)
-            m[2 * h] = __ballot_sync(0xffffffffu, in && (q1a <= rl[2 * h] || q2a <= rl[2 * h]));
-            m[2 * h + 1] = __ballot_sync(0xffffffffu, in && (q1b <= rl[2 * h + 1] || q2b <= rl[2 * h + 1]));
-          }
+        for (int h = 0; h < 2; ++h) {
+          const float f0 = py0 + (float)(2 * h) * th, f1 = f0 + th;
+          unpack2(add2(pack2(f0, f1), nmu), y0[2 * h], y0[2 * h + 1]);
+          unpack2(add2(pack2(fminf(f0 + (th - 1.0f), y_last), fminf(f1 + (th - 1.0f), y_last)), nmu),
+                  y1[2 * h], y1[2 * h + 1]);
+          const float na = clampf(0.0f, y0[2 * h], y1[2 * h]);
+          const float nb = clampf(0.0f, y0[2 * h + 1], y1[2 * h + 1]);
+          const f2 n = pack2(na, nb), num = mul2(nb2, n);
+          unpack2(fast ? div2(num, nd, y2) : div2_ieee(num, nd), rz[2 * h], rz[2 * h + 1]);
+          float wa, wb;
+          unpack2(mul2(mul2(cc2, n), n), wa, wb);
+          yn[2 * h] = pack2(na, na);
+          yn[2 * h + 1] = pack2(nb, nb);
+          rw[2 * h] = pack2(wa, wa);
+          rw[2 * h + 1] = pack2(wb, wb);
         }
-        if (lane == 0) *reinterpret_cast<uint4*>(sm + 4 * k) = make_uint4(m[0], m[1], m[2], m[3]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          rl[k] = bx.valid && ty0 + k >= bx.y0 && ty0 + k <= bx.y1 ? lim : nan;
+      }
+      const f2 nmu = pack2(-bx.mu_x, -bx.mu_x), nd = pack2(-cc_, -cc_), y2 = pack2(yc, yc);
+#pragma unroll 1
+      for (uint32_t k = 0; k < 8; k += 2) {
+        const uint32_t tx = tx0 + k;
+        const bool in0 = tx >= bx.x0 && tx <= bx.x1, in1 = tx + 1 >= bx.x0 && tx + 1 <= bx.x1;
+        const float f0 = px0 + (float)k * tw, f1 = f0 + tw;
+        float x0a, x0b, x1a, x1b;
+        unpack2(add2(pack2(f0, f1), nmu), x0a, x0b);
+        unpack2(add2(pack2(fminf(f0 + (tw - 1.0f), x_last), fminf(f1 + (tw - 1.0f), x_last)), nmu), x1a,
+                x1b);
+        const f2 xn = pack2(clampf(0.0f, x0a, x1a), clampf(0.0f, x0b, x1b));
+        const f2 num = mul2(nb2, xn);
+        float cza, czb;
+        unpack2(fast ? div2(num, nd, y2) : div2_ieee(num, nd), cza, czb);
+        const f2 cw = fma2(mul2(ca2, xn), xn, nz);
+        const f2 cp = mul2(cb22, xn);
+        uint32_t m0[4], m1[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const f2 y = pack2(clampf(cza, y0[r], y1[r]), clampf(czb, y0[r], y1[r]));
+          const f2 q1 = add2(add2(cw, fma2(cp, y, nz)), fma2(mul2(cc2, y), y, nz));
+          const f2 x = pack2(clampf(rz[r], x0a, x1a), clampf(rz[r], x0b, x1b));
+          const f2 q2 = add2(add2(fma2(mul2(ca2, x), x, nz), fma2(mul2(cb22, x), yn[r], nz)), rw[r]);
+          float q1a, q1b, q2a, q2b;
+          unpack2(q1, q1a, q1b);
+          unpack2(q2, q2a, q2b);
+          // fminf(q1, q2) <= limit: either is (a NaN never is)
+          m0[r] = __ballot_sync(0xffffffffu, in0 && (q1a <= rl[r] || q2a <= rl[r]));
+          m1[r] = __ballot_sync(0xffffffffu, in1 && (q1b <= rl[r] || q2b <= rl[r]));
+        }
+        if (lane == 0) {
+          *reinterpret_cast<uint4*>(sm + 4 * k) = make_uint4(m0[0], m0[1], m0[2], m0[3]);
+          *reinterpret_cast<uint4*>(sm + 4 * k + 4) = make_uint4(m1[0], m1[1], m1[2], m1[3]);
+        }
       }
       __syncwarp();
       // lane t holds tile t (row-major in the block)
@@ -445,10 +481,20 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
         if (lane >= o) incl += y;
       }
       const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-      uint32_t at_s = incl - n;
-      s_delta[warp][lane] = p - at_s;
-      for (uint32_t m = m0; m; m &= m - 1u) stage[at_s++] = (uint16_t)((lane << 6) | (__ffs(m) - 1));
-      for (uint32_t m = m1; m; m &= m - 1u) stage[at_s++] = (uint16_t)((lane << 6) | (31 + __ffs(m)));
+      s_delta[warp][lane] = p - (incl - n);
+      // from the highest bit down, backwards from the tile's end
+      uint16_t* at_s = stage + incl;
+      const uint32_t tile = (uint32_t)lane << 6;
+      for (uint32_t m = m1; m;) {
+        const uint32_t bit = 31u - __clz(m);
+        m ^= 1u << bit;
+        *--at_s = (uint16_t)(tile + 32u + bit);
+      }
+      for (uint32_t m = m0; m;) {
+        const uint32_t bit = 31u - __clz(m);
+        m ^= 1u << bit;
+        *--at_s = (uint16_t)(tile + bit);
+      }
       __syncwarp();
       for (uint32_t k = lane; k < total; k += 32) {
         const uint32_t e = stage[k];

@@ -82,23 +82,6 @@ __device__ __forceinline__ float div_rcp64(float n, float d, double y) {
   return r;
 }
 
-// n / d correctly rounded to binary32 from y = RN(1 / d), by Markstein's
-// division (IBM J. Res. Dev. 34(1), 1990): the first step makes q faithful,
-// and from a faithful q and a correctly rounded reciprocal the second gives
-// the correctly rounded quotient, as long as nothing under- or overflows.
-// `ok` says that d lies in [2^-40, 2^20] and |n| below 2^63; a quotient below
-// 2^-60 in magnitude (other than zero) takes the division itself. The sign of
-// a zero is not kept. Checked against n / d on 3 x 10^9 operand pairs; 9
-// instructions of the product pipe's rate instead of the two conversions and
-// the binary64 product of div_rcp64, which hold the conversion pipe.
-__device__ __forceinline__ float div_rcp32(float n, float d, float y, bool ok) {
-  const float q = __fmul_rn(n, y);
-  const float q1 = __fmaf_rn(__fmaf_rn(-d, q, n), y, q);
-  float r = __fmaf_rn(__fmaf_rn(-d, q1, n), y, q1);
-  if (!ok || (!(fabsf(q) >= 0x1p-60f) && n != 0.0f)) r = div_ieee(n, d);
-  return r;
-}
-
 // Column terms of a splat's tile column tx (the parts of the test that depend
 // on the column alone): x edges, the y minimiser at the column's nearest x
 // (before its clamp to the row), a x_near^2.

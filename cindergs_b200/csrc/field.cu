@@ -127,7 +127,7 @@ cudaError_t FieldState::init(uint32_t nv, const float* rest_v4, uint64_t seed, c
   FIELD_TRY(proj_rest.ensure((size_t)kFieldProj * 4));
   FIELD_TRY(loss.ensure(16));
   FIELD_TRY(status.ensure(16));
-  FIELD_TRY(wT.ensure((size_t)kFieldHid * std::max<uint32_t>(ldV, kFieldHid) * 2));
+  FIELD_TRY(wT.ensure((size_t)kFieldHid * (3 * kFieldHid + ldV) * 2));
   FIELD_TRY(cudaMemsetAsync(m1.p, 0, (size_t)o * 4, s));
   FIELD_TRY(cudaMemsetAsync(m2.p, 0, (size_t)o * 4, s));
   FIELD_TRY(cudaMemsetAsync(g32.p, 0, (size_t)o * 4, s));
@@ -136,7 +136,7 @@ cudaError_t FieldState::init(uint32_t nv, const float* rest_v4, uint64_t seed, c
   FIELD_TRY(cudaMemcpyAsync(rest_d.p, rest_v4, (size_t)nv * 16, cudaMemcpyHostToDevice, s));
   step = 0;
   FIELD_TRY(cudaMemcpyAsync(p32.p, h.data(), (size_t)o * 4, cudaMemcpyHostToDevice, s));
-  FIELD_TRY(launch_transpose_f32(p32.as<float>(), 1, o, o, pb.as<__nv_bfloat16>(), 1, s));
+  FIELD_TRY(refresh(s));
   return cudaStreamSynchronize(s);  // h goes out of scope
 }
 
@@ -157,46 +157,59 @@ FieldNet FieldState::net() const {
   return n;
 }
 
-cudaError_t FieldState::ensure_batch(uint32_t B) {
-  if (B <= Bcap) return cudaSuccess;
+cudaError_t FieldState::ensure_batch(uint32_t B, bool train) {
   const size_t b = B, H = kFieldHid;
-  FIELD_TRY(x.ensure(b * 12));
-  FIELD_TRY(wt.ensure(b * ldV * 4));
-  FIELD_TRY(a0.ensure(b * kFieldIn * 2));
-  for (int l = 0; l < 4; ++l) {
-    FIELD_TRY(pre[l].ensure(b * H * 4));
-    FIELD_TRY(h[l].ensure(b * H * 2));
+  if (B > Bcap) {
+    FIELD_TRY(x.ensure(b * 12));
+    FIELD_TRY(idx.ensure(b * 4));
+    FIELD_TRY(a0.ensure(b * kFieldIn * 2));
+    for (int l = 0; l < 4; ++l) {
+      FIELD_TRY(pre[l].ensure(b * H * 4));
+      FIELD_TRY(h[l].ensure(b * H * 2));
+    }
+    FIELD_TRY(z.ensure(b * ldV * 4));
+    Bcap = B;
   }
-  FIELD_TRY(z.ensure(b * ldV * 4));
-  FIELD_TRY(dz.ensure(b * ldV * 4));
-  FIELD_TRY(dzb.ensure(b * ldV * 2));
-  FIELD_TRY(dzT.ensure((size_t)ldV * b * 2));
-  FIELD_TRY(hT.ensure(H * b * 2));
-  FIELD_TRY(dpre.ensure(b * H * 4));
-  FIELD_TRY(dpreb.ensure(b * H * 2));
-  FIELD_TRY(dpreT.ensure(H * b * 2));
-  FIELD_TRY(dh.ensure(b * H * 4));
-  FIELD_TRY(gemm_ws.ensure((size_t)16 * std::max<uint32_t>(ldV, kFieldHid) * H * 4));
-  Bcap = B;
+  if (train && B > Btrain) {
+    FIELD_TRY(dzb.ensure(b * ldV * 2));
+    for (int l = 0; l < 2; ++l) FIELD_TRY(dpreb[l].ensure(b * H * 2));
+    for (int l = 0; l < 5; ++l) {
+      FIELD_TRY(inT[l].ensure((l == 0 ? kFieldIn : H) * b * 2));
+      FIELD_TRY(dT[l].ensure((l == 4 ? ldV : H) * b * 2));
+      if (l < 4) FIELD_TRY(dpre[l].ensure(b * H * 4));
+    }
+    FIELD_TRY(dz.ensure(b * ldV * 4));
+    FIELD_TRY(gemm_ws.ensure((size_t)16 * (H * kFieldIn + 3 * H * H + (size_t)V * H) * 4));
+    Btrain = B;
+  }
   return cudaSuccess;
+}
+
+void FieldState::transposed(__nv_bfloat16* (&w)[4]) const {
+  for (int l = 0; l < 4; ++l) w[l] = wT.as<__nv_bfloat16>() + (size_t)l * kFieldHid * kFieldHid;
+}
+
+cudaError_t FieldState::refresh(cudaStream_t s) {
+  __nv_bfloat16* w[4];
+  transposed(w);
+  return launch_field_refresh(off, V, ldV, p32.as<float>(), pb.as<__nv_bfloat16>(), w, s);
 }
 
 cudaError_t FieldState::forward(const float* points, const float* target, uint32_t n, uint32_t B,
                                 uint32_t seed, const float4* rest_verts, float lambda,
                                 cudaStream_t s) {
-  FIELD_TRY(ensure_batch(B));
+  const bool train = target != nullptr;
+  FIELD_TRY(ensure_batch(B, train));
   FieldBatch fb{};
   fb.points = points;
-  fb.target = target;
   fb.n = n;
-  fb.V = V;
   fb.B = B;
-  fb.ldw = ldV;
   fb.seed = seed;
   fb.enc = enc_d.as<float>();
   fb.x = x.as<float>();
-  fb.wt = wt.as<float>();
+  fb.idx = idx.as<uint32_t>();
   fb.a0 = a0.as<__nv_bfloat16>();
+  fb.a0T = train ? inT[0].as<__nv_bfloat16>() : nullptr;
   FIELD_TRY(launch_field_gather(fb, s));
   const FieldNet nt = net();
   const __nv_bfloat16* W[4] = {nt.W1b, nt.W2b, nt.W3b, nt.W4b};
@@ -215,6 +228,8 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
     g.bias = bias[l];
     g.D = h[l].as<__nv_bfloat16>();
     g.ldd = kFieldHid;
+    g.DT = train ? inT[l + 1].as<__nv_bfloat16>() : nullptr;
+    g.ldt = B;
     FIELD_TRY(launch_gemm_nt(g, kEpiBiasSilu, s));
   }
   GemmArgs g{};
@@ -232,110 +247,98 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
   if (!target) return cudaSuccess;
   FieldLoss fl{};
   fl.z = z.as<float>();
-  fl.wt = wt.as<float>();
+  fl.target = target;
+  fl.idx = idx.as<uint32_t>();
   fl.x = x.as<float>();
   fl.verts = rest_verts;
   fl.B = B;
   fl.V = V;
   fl.ldz = ldV;
-  fl.ldw = ldV;
   fl.lambda = lambda;
   fl.s2 = scale * scale;
   std::memcpy(fl.M, M.m, 64);
-  fl.dz = dz.as<float>();
   fl.dzb = dzb.as<__nv_bfloat16>();
+  fl.dzT = dT[4].as<__nv_bfloat16>();
+  fl.dz = dz.as<float>();
   fl.loss = loss.as<float>();
   return launch_field_loss(fl, s);
 }
 
 cudaError_t FieldState::backward(uint32_t B, cudaStream_t s) {
   if (B % 8) return cudaErrorInvalidValue;  // transposed operands have row length B
-  const FieldNet nt = net();
-  float* g = g32.as<float>();
-  __nv_bfloat16* wTb = wT.as<__nv_bfloat16>();
-  // output layer: dW5 = dz^T h4, db5 = sum_rows dz, dh4 = dz W5
-  FIELD_TRY(launch_transpose_f32(dz.as<float>(), B, V, ldV, dzT.as<__nv_bfloat16>(), B, s));
-  FIELD_TRY(launch_transpose_bf16(h[3].as<__nv_bfloat16>(), B, kFieldHid, kFieldHid,
-                                  hT.as<__nv_bfloat16>(), B, s));
-  GemmArgs gw{};
-  gw.status = status.as<uint32_t>();
-  gw.ws = gemm_ws.as<float>();
-  gw.ws_floats = gemm_ws.cap / 4;
-  gw.A = dzT.as<__nv_bfloat16>();
-  gw.lda = B;
-  gw.B = hT.as<__nv_bfloat16>();
-  gw.ldb = B;
-  gw.M = V;
-  gw.N = kFieldHid;
-  gw.K = B;
-  gw.C = g + off[kW5];
-  gw.ldc = kFieldHid;
-  FIELD_TRY(launch_gemm_nt(gw, kEpiF32, s));
-  FIELD_TRY(launch_colsum(dz.as<float>(), B, V, ldV, g + off[kB5], s));
-  FIELD_TRY(launch_transpose_bf16(nt.W5b, V, kFieldHid, kFieldHid, wTb, ldV, s));
-  GemmArgs gd{};
-  gd.status = status.as<uint32_t>();
-  gd.A = dzb.as<__nv_bfloat16>();
-  gd.lda = ldV;
-  gd.B = wTb;
-  gd.ldb = ldV;
-  gd.M = B;
-  gd.N = kFieldHid;
-  gd.K = V;
-  gd.C = dh.as<float>();
-  gd.ldc = kFieldHid;
-  FIELD_TRY(launch_gemm_nt(gd, kEpiF32, s));
-  const __nv_bfloat16* Wl[4] = {nt.W1b, nt.W2b, nt.W3b, nt.W4b};
-  const int wk[4] = {kW1, kW2, kW3, kW4}, bk[4] = {kB1, kB2, kB3, kB4};
+  __nv_bfloat16* w[4];
+  transposed(w);
+  // dL/dpre of layer l = (dL/dz or dL/dpre of the layer above) W silu'(pre_l)
   for (int l = 3; l >= 0; --l) {
-    FIELD_TRY(launch_silu_back(B * kFieldHid, dh.as<float>(), pre[l].as<float>(), dpre.as<float>(),
-                               dpreb.as<__nv_bfloat16>(), s));
-    FIELD_TRY(launch_transpose_f32(dpre.as<float>(), B, kFieldHid, kFieldHid,
-                                   dpreT.as<__nv_bfloat16>(), B, s));
-    const uint32_t kin = l == 0 ? kFieldIn : kFieldHid;
-    const __nv_bfloat16* in = l == 0 ? a0.as<__nv_bfloat16>() : h[l - 1].as<__nv_bfloat16>();
-    FIELD_TRY(launch_transpose_bf16(in, B, kin, kin, hT.as<__nv_bfloat16>(), B, s));
-    GemmArgs gl{};
-    gl.status = status.as<uint32_t>();
-    gl.ws = gemm_ws.as<float>();
-    gl.ws_floats = gemm_ws.cap / 4;
-    gl.A = dpreT.as<__nv_bfloat16>();
-    gl.lda = B;
-    gl.B = hT.as<__nv_bfloat16>();
-    gl.ldb = B;
-    gl.M = kFieldHid;
-    gl.N = kin;
-    gl.K = B;
-    gl.C = g + off[wk[l]];
-    gl.ldc = kin;
-    FIELD_TRY(launch_gemm_nt(gl, kEpiF32, s));
-    FIELD_TRY(launch_colsum(dpre.as<float>(), B, kFieldHid, kFieldHid, g + off[bk[l]], s));
-    if (l > 0) {
-      FIELD_TRY(launch_transpose_bf16(Wl[l], kFieldHid, kFieldHid, kFieldHid, wTb, kFieldHid, s));
-      GemmArgs gh{};
-      gh.status = status.as<uint32_t>();
-      gh.A = dpreb.as<__nv_bfloat16>();
-      gh.lda = kFieldHid;
-      gh.B = wTb;
-      gh.ldb = kFieldHid;
-      gh.M = B;
-      gh.N = kFieldHid;
-      gh.K = kFieldHid;
-      gh.C = dh.as<float>();
-      gh.ldc = kFieldHid;
-      FIELD_TRY(launch_gemm_nt(gh, kEpiF32, s));
-    }
+    GemmArgs g{};
+    g.status = status.as<uint32_t>();
+    g.A = l == 3 ? dzb.as<__nv_bfloat16>() : dpreb[(l + 1) & 1].as<__nv_bfloat16>();
+    g.lda = l == 3 ? ldV : kFieldHid;
+    g.K = l == 3 ? V : kFieldHid;
+    g.B = w[l];
+    g.ldb = g.lda;
+    g.M = B;
+    g.N = kFieldHid;
+    g.pre = pre[l].as<float>();
+    g.C = dpre[l].as<float>();
+    g.ldc = kFieldHid;
+    g.D = l > 0 ? dpreb[l & 1].as<__nv_bfloat16>() : nullptr;
+    g.ldd = kFieldHid;
+    g.DT = dT[l].as<__nv_bfloat16>();
+    g.ldt = B;
+    FIELD_TRY(launch_gemm_nt(g, kEpiBack, s));
   }
-  return cudaSuccess;
+  // dW_l = (dL/dpre_l or dL/dz)^T (input of the layer), db_l = their column sums
+  GemmBatch gb{};
+  gb.splits = grad_splits(B);
+  float* ws = gemm_ws.as<float>();
+  for (int l = 0; l < 5; ++l) {
+    GemmArgs& g = gb.g[l];
+    g.status = status.as<uint32_t>();
+    g.A = dT[l].as<__nv_bfloat16>();
+    g.B = inT[l].as<__nv_bfloat16>();
+    g.lda = g.ldb = g.K = B;
+    g.M = l == 4 ? V : kFieldHid;
+    g.N = l == 0 ? kFieldIn : kFieldHid;
+    g.C = ws;
+    ws += (size_t)16 * g.M * g.N;
+    gb.first[l + 1] = gb.first[l] + (g.M + 127) / 128 * ((g.N + 63) / 64);
+    gb.sum[l] = l == 4 ? dz.as<float>() : dpre[l].as<float>();
+    gb.sum_n[l] = g.M;
+    gb.sum_ld[l] = l == 4 ? ldV : kFieldHid;
+    gb.sum_out[l] = g32.as<float>() + off[2 * l + 1];
+  }
+  return launch_gemm_grads(gb, s);
 }
 
-cudaError_t FieldState::adam(float lr, cudaStream_t s) {
-  ++step;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)step)));
-  const float c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)step)));
-  return launch_adam(total(), p32.as<float>(), g32.as<float>(), m1.as<float>(), m2.as<float>(),
-                     pb.as<__nv_bfloat16>(), lr, b1, b2, 1e-8f, c1, c2, s);
+cudaError_t FieldState::update(uint32_t B, float lr, cudaStream_t s) {
+  FieldUpdate u{};
+  for (int k = 0; k <= kFieldParams; ++k) u.off[k] = off[k];
+  u.V = V;
+  u.ldV = ldV;
+  u.splits = grad_splits(B);
+  const float* ws = gemm_ws.as<float>();
+  for (int l = 0; l < 5; ++l) {
+    u.ws[l] = ws;
+    ws += (size_t)16 * (l == 4 ? V : kFieldHid) * (l == 0 ? kFieldIn : kFieldHid);
+  }
+  u.p = p32.as<float>();
+  u.g = g32.as<float>();
+  u.m = m1.as<float>();
+  u.v = m2.as<float>();
+  u.pb = pb.as<__nv_bfloat16>();
+  transposed(u.wT);
+  u.adam = lr > 0.0f ? 1 : 0;
+  if (u.adam) {
+    ++step;
+    u.lr = lr;
+    u.b1 = 0.9f;
+    u.b2 = 0.999f;
+    u.eps = 1e-8f;
+    u.c1 = (float)(1.0 / (1.0 - std::pow(0.9, (double)step)));
+    u.c2 = (float)(1.0 / (1.0 - std::pow(0.999, (double)step)));
+  }
+  return launch_field_update(u, s);
 }
 
 cudaError_t FieldState::eval(uint32_t n, const float* points, float* w, cudaStream_t s) {

@@ -36,10 +36,12 @@ struct FieldState {
   float scale = 1.0f;       // s: half of the largest rest-cage extent
   FieldMat M{};             // (Vb Vb^T)^-1, Vb = [1; rest vertices]
   uint32_t step = 0;        // Adam steps taken
-  FieldBuf p32, g32, m1, m2, pb, enc_d, M_d, rest_d, proj, proj_rest, loss, wT, status;
+  FieldBuf p32, g32, m1, m2, pb, enc_d, M_d, rest_d, proj, proj_rest, loss, wT, status;  // wT: W2..W5 transposed
   // training batch (B rows)
-  uint32_t Bcap = 0;
-  FieldBuf x, wt, a0, pre[4], h[4], z, dz, dzb, dzT, hT, dpre, dpreb, dpreT, dh;
+  uint32_t Bcap = 0, Btrain = 0;
+  // inT: the transposed inputs of layers 1..5 (features, then h); dT: the
+  // transposed dL/dpre of layers 1..4 and dL/dz; dpre, dz: the same in fp32
+  FieldBuf x, idx, a0, pre[4], h[4], z, dz, dzb, dpre[4], dpreb[2], inT[5], dT[5];
   FieldBuf gemm_ws;  // split-K partial sums of the weight gradients (K = batch)
 
   uint32_t total() const { return off[kFieldParams]; }
@@ -48,14 +50,18 @@ struct FieldState {
   // output weights N(0, 1e-6), output biases 1/V (uniform weights).
   cudaError_t init(uint32_t V, const float* rest_v4, uint64_t seed, cudaStream_t s);
   FieldNet net() const;
-  cudaError_t ensure_batch(uint32_t B);
+  cudaError_t ensure_batch(uint32_t B, bool train);
   // Forward over a batch (rows r -> points as FieldBatch::seed says), with
-  // the loss and dL/dz when target is given, and the backward pass into g32
-  // when backward is set. loss[0..1] accumulate in `loss`.
+  // the loss and dL/dz when target is given. loss[0..1] accumulate in `loss`.
   cudaError_t forward(const float* points, const float* target, uint32_t n, uint32_t B,
                       uint32_t seed, const float4* rest_verts, float lambda, cudaStream_t s);
+  // Products of the backward pass; update() turns their partial sums into the
+  // gradients and, with lr > 0, takes an Adam step.
   cudaError_t backward(uint32_t B, cudaStream_t s);
-  cudaError_t adam(float lr, cudaStream_t s);
+  cudaError_t update(uint32_t B, float lr, cudaStream_t s);
+  // bf16 copy (and the transposed weights) from the fp32 parameters
+  cudaError_t refresh(cudaStream_t s);
+  void transposed(__nv_bfloat16* (&w)[4]) const;
   // Final (projected) weights of n points [n*3] into w [n*V].
   cudaError_t eval(uint32_t n, const float* points, float* w, cudaStream_t s);
   // Per-frame projection of the output layer for current vertices [V]

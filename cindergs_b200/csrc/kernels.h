@@ -81,7 +81,10 @@ cudaError_t launch_mvc_residual(uint32_t nb, const uint32_t* list, const float4*
 constexpr int kFieldBands = 8;
 constexpr int kFieldIn = 64;    // 3 + 6 * bands, zero-padded
 constexpr int kFieldHid = 128;
-constexpr int kEpiF32 = 0, kEpiBias = 1, kEpiBiasSilu = 2;
+// epilogues of the training GEMMs: bias (C), bias and SiLU (C, D and its
+// transpose), SiLU slope of the layer below (C, D and its transpose), split
+// partial sums
+constexpr int kEpiBias = 1, kEpiBiasSilu = 2, kEpiBack = 3, kEpiSplit = 4;
 // per-frame projection: Pc (128 x 3), pc (3), A3 (3 x 3)
 constexpr int kFieldProj = 3 * kFieldHid + 3 + 9;
 struct FieldMat {  // M = (Vb Vb^T)^-1, row-major 4 x 4
@@ -92,40 +95,70 @@ struct FieldNet {  // device pointers into one parameter block
   const __nv_bfloat16 *W1b, *W2b, *W3b, *W4b, *W5b;
   const float *b1, *b2, *b3, *b4, *b5;
 };
-struct GemmArgs {  // C = A B^T (+ bias), D = bf16(silu(C)); tcgen05 (mvc_field_tc.cu)
+struct GemmArgs {  // C = A B^T; tcgen05 (mvc_field_tc.cu)
   const __nv_bfloat16* A;
   const __nv_bfloat16* B;
   uint32_t M, N, K, lda, ldb;
-  float* C;
+  float* C;              // fp32 result (+ bias, times silu'(pre)), or the splits' [z][M][N]
   uint32_t ldc;
-  const float* bias;
-  __nv_bfloat16* D;
+  const float* bias;     // [N]
+  __nv_bfloat16* D;      // bf16(silu(C)), or bf16(C silu'(pre)); or null
   uint32_t ldd;
+  __nv_bfloat16* DT;     // D transposed [N][ldt], or null
+  uint32_t ldt;
+  const float* pre;      // [M][ldc] (kEpiBack)
   uint32_t* status;      // kStatusBarrierTimeout / kStatusPoisoned on a failed wait, or null
-  float* ws;             // split-K partial sums (F32 epilogue), or null: no split
-  size_t ws_floats;
 };
+// The weight gradients of all layers in one launch: problem p's tiles are
+// [first[p], first[p + 1]) of 128 x 64, K split into `splits` ranges; and the
+// bias gradients, the column sums over the batch's rows of sum[p] [K][ld].
+constexpr int kGradProblems = 5;
+struct GemmBatch {
+  GemmArgs g[kGradProblems];
+  uint32_t first[kGradProblems + 1];
+  uint32_t splits;
+  const float* sum[kGradProblems];
+  float* sum_out[kGradProblems];
+  uint32_t sum_n[kGradProblems], sum_ld[kGradProblems];
+};
+uint32_t grad_splits(uint32_t B);  // ranges of K = B
 struct FieldBatch {
   const float* points;   // [n*3]
-  const float* target;   // [n*V] exact weights or null
-  uint32_t n, V, B, ldw;
+  uint32_t n, B;
   uint32_t seed;         // 0: rows r % n in order
   const float* enc;      // [4] centre xyz, 1/s
   float* x;              // [B*3]
-  float* wt;             // [B*ldw]
+  uint32_t* idx;         // [B] the point of each row
   __nv_bfloat16* a0;     // [B*64]
+  __nv_bfloat16* a0T;    // [64*B] or null
 };
 struct FieldLoss {
   const float* z;        // [B*ldz]
-  const float* wt;       // [B*ldw]
+  const float* target;   // [n*V] exact weights
+  const uint32_t* idx;   // [B] row -> point
   const float* x;        // [B*3]
   const float4* verts;   // [V] rest vertices
-  uint32_t B, V, ldz, ldw;
+  uint32_t B, V, ldz;
   float lambda, s2;
   float M[16];           // (Vb Vb^T)^-1 of the rest cage
-  float* dz;             // [B*ldz]
   __nv_bfloat16* dzb;    // [B*ldz]
+  __nv_bfloat16* dzT;    // [V*B]
+  float* dz;             // [B*ldz]
   float* loss;           // [2] accumulated (weight term, residual term)
+};
+constexpr uint32_t kLossRows = 16;  // rows of one loss block
+// Weight gradients from the split partial sums, and Adam on all gradients
+// (adam = 0: gradients only); refreshes the bf16 weights and the transposed
+// copies that the backward products read.
+struct FieldUpdate {
+  uint32_t off[11];      // parameter offsets (FieldParam), total
+  uint32_t V, ldV, splits;
+  const float* ws[5];    // W1..W5 partial sums [splits][rows][cols]
+  float *p, *g, *m, *v;  // g: the bias gradients in, all gradients out
+  __nv_bfloat16* pb;
+  __nv_bfloat16* wT[4];  // W2..W4 transposed [128][128], W5 transposed [128][ldV]
+  int adam;
+  float lr, b1, b2, eps, c1, c2;
 };
 struct FieldInfer {
   FieldNet net;
@@ -145,18 +178,12 @@ struct FieldInfer {
 };
 cudaError_t launch_field_gather(const FieldBatch& b, cudaStream_t s);
 cudaError_t launch_gemm_nt(const GemmArgs& g, int epi, cudaStream_t s);
-cudaError_t launch_transpose_f32(const float* in, uint32_t R, uint32_t C, uint32_t ldi,
-                                 __nv_bfloat16* out, uint32_t ldo, cudaStream_t s);
-cudaError_t launch_transpose_bf16(const __nv_bfloat16* in, uint32_t R, uint32_t C, uint32_t ldi,
-                                  __nv_bfloat16* out, uint32_t ldo, cudaStream_t s);
+cudaError_t launch_gemm_grads(const GemmBatch& g, cudaStream_t s);
+// out = bf16(in), and W2..W5 transposed into wT (null: not wanted)
+cudaError_t launch_field_refresh(const uint32_t* off, uint32_t V, uint32_t ldV, const float* p,
+                                 __nv_bfloat16* pb, __nv_bfloat16* const* wT, cudaStream_t s);
 cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s);
-cudaError_t launch_silu_back(uint32_t n, const float* da, const float* pre, float* dpre,
-                             __nv_bfloat16* dpreb, cudaStream_t s);
-cudaError_t launch_colsum(const float* g, uint32_t B, uint32_t N, uint32_t ld, float* out,
-                          cudaStream_t s);
-cudaError_t launch_adam(uint32_t n, float* p, const float* g, float* m, float* v,
-                        __nv_bfloat16* pb, float lr, float b1, float b2, float eps, float c1,
-                        float c2, cudaStream_t s);
+cudaError_t launch_field_update(const FieldUpdate& u, cudaStream_t s);
 // verts null: the network's own rest position (no linear-precision
 // projection); otherwise the projected weights on current vertices verts.
 cudaError_t launch_field_project(const FieldNet& net, uint32_t V, const float4* rest,

@@ -43,11 +43,6 @@ namespace {
 constexpr int kIn = kFieldIn;    // 64 features
 constexpr int kHid = kFieldHid;  // 128
 
-__device__ __forceinline__ float sigmoid_fast(float x) { return 1.0f / (1.0f + __expf(-x)); }
-__device__ __forceinline__ float silu_grad(float x) {
-  const float s = sigmoid_fast(x);
-  return s * (1.0f + x * (1.0f - s));
-}
 
 // Feature j of x^ (value) and its derivatives with respect to x (chain factor
 // 1/s), for j in [0, 64).
@@ -83,44 +78,73 @@ __device__ __forceinline__ uint32_t mix32(uint64_t z) {
 }
 
 // Batch gather and features: row r uses point idx = mix(seed, r) % n (or r
-// when seed is 0); writes x [B*3], target weights [B x ldw] and features
-// A0 [B x 64] (bf16).
-__global__ void k_field_gather(FieldBatch fb) {
-  const uint32_t r = blockIdx.x;
-  if (r >= fb.B) return;
-  const uint32_t idx = fb.seed ? mix32(((uint64_t)fb.seed << 32) | r) % fb.n : r % fb.n;
-  __shared__ float xh[3];
-  if (threadIdx.x < 3) {
-    const float x = fb.points[3 * (size_t)idx + threadIdx.x];
-    fb.x[3 * (size_t)r + threadIdx.x] = x;
-    xh[threadIdx.x] = (x - fb.enc[threadIdx.x]) * fb.enc[3];
+// when seed is 0); writes x [B*3], idx and features A0 [B x 64] (bf16) and
+// their transpose. 32 rows per block, so that the transpose is written 64
+// bytes at a time.
+constexpr int kGatherRows = 32;
+__global__ void __launch_bounds__(256) k_field_gather(FieldBatch fb) {
+  __shared__ float xh[kGatherRows][3];
+  __shared__ __nv_bfloat16 tile[kIn][kGatherRows + 2];
+  const uint32_t r0 = blockIdx.x * kGatherRows;
+  if (threadIdx.x < kGatherRows) {
+    const uint32_t r = r0 + threadIdx.x;
+    if (r < fb.B) {
+      const uint32_t idx = fb.seed ? mix32(((uint64_t)fb.seed << 32) | r) % fb.n : r % fb.n;
+      fb.idx[r] = idx;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const float x = fb.points[3 * (size_t)idx + d];
+        fb.x[3 * (size_t)r + d] = x;
+        xh[threadIdx.x][d] = (x - fb.enc[d]) * fb.enc[3];
+      }
+    }
   }
   __syncthreads();
-  if (fb.target)
-    for (uint32_t j = threadIdx.x; j < fb.V; j += blockDim.x)
-      fb.wt[(size_t)r * fb.ldw + j] = fb.target[(size_t)idx * fb.V + j];
-  for (int j = threadIdx.x; j < kIn; j += blockDim.x) {
+  for (int k = threadIdx.x; k < kGatherRows * kIn; k += 256) {
+    const int q = k / kIn, j = k % kIn;
+    if (r0 + q >= fb.B) break;
     float f, df[3];
-    feature(j, xh, fb.enc[3], f, df);
-    fb.a0[(size_t)r * kIn + j] = __float2bfloat16_rn(f);
+    feature(j, xh[q], fb.enc[3], f, df);
+    const __nv_bfloat16 v = __float2bfloat16_rn(f);
+    fb.a0[(size_t)(r0 + q) * kIn + j] = v;
+    tile[j][q] = v;
+  }
+  if (!fb.a0T) return;
+  __syncthreads();
+  for (int k = threadIdx.x; k < kGatherRows * kIn; k += 256) {
+    const int j = k / kGatherRows, q = k % kGatherRows;
+    if (r0 + q < fb.B) fb.a0T[(size_t)j * fb.B + r0 + q] = tile[j][q];
   }
 }
 
-// out [C x R] bf16 = transpose of in [R x C] (fp32 or bf16).
-template <typename T>
-__global__ void k_transpose(const T* __restrict__ in, uint32_t R, uint32_t C, uint32_t ldi,
-                            __nv_bfloat16* __restrict__ out, uint32_t ldo) {
-  __shared__ float tile[32][33];
-  const uint32_t c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const uint32_t r = r0 + k, c = c0 + threadIdx.x;
-    tile[k][threadIdx.x] = (r < R && c < C) ? (float)in[(size_t)r * ldi + c] : 0.0f;
+// bf16 copy of the parameters, and W2..W5 transposed for the products that
+// carry dL/dh down a layer (wT null: not wanted).
+struct RefreshArgs {
+  uint32_t off[11];
+  uint32_t V, ldV;
+  const float* p;
+  __nv_bfloat16* pb;
+  __nv_bfloat16* wT[4];
+};
+// parameter i's transposed copy
+__device__ __forceinline__ void put_transposed(const uint32_t* off, uint32_t ldV,
+                                               __nv_bfloat16* const* wT, uint32_t i,
+                                               __nv_bfloat16 w) {
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const uint32_t o = off[2 * (l + 1)], e = off[2 * (l + 1) + 1];
+    if (i >= o && i < e) {
+      const uint32_t k = i - o, r = k / kHid, c = k % kHid, ld = l == 3 ? ldV : (uint32_t)kHid;
+      if (r < ld) wT[l][(size_t)c * ld + r] = w;
+    }
   }
-  __syncthreads();
-  for (int k = threadIdx.y; k < 32; k += blockDim.y) {
-    const uint32_t c = c0 + k, r = r0 + threadIdx.x;
-    if (c < C && r < R) out[(size_t)c * ldo + r] = __float2bfloat16_rn(tile[threadIdx.x][k]);
-  }
+}
+__global__ void k_field_refresh(RefreshArgs a) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.off[10]) return;
+  const __nv_bfloat16 w = __float2bfloat16_rn(a.p[i]);
+  a.pb[i] = w;
+  if (a.wT[0]) put_transposed(a.off, a.ldV, a.wT, i, w);
 }
 
 // Sums of K values over the block (blockDim.x a multiple of 32, at most 1024);
@@ -151,118 +175,187 @@ __device__ __forceinline__ void lp_correction(const float* M, const float (&r)[3
   for (int a = 0; a < 4; ++a) u[a] = M[4 * a + 1] * r[0] + M[4 * a + 2] * r[1] + M[4 * a + 3] * r[2];
 }
 
+// Sums over a row held by one warp: v[k][c] is the partial sum of value k over
+// the columns j with j % 128 = 32 c + lane. Each group of 32 is added by a
+// butterfly, the four groups in order.
+template <int K>
+__device__ __forceinline__ void row_sums(float (&v)[K][4], float (&out)[K]) {
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k][c] += __shfl_xor_sync(0xffffffffu, v[k][c], o);
+    float t = 0.0f;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) t += v[k][c];
+    out[k] = t;
+  }
+}
+
 // Loss and dL/dz per batch row. w0 = z + (1 - sum z) / V; r = sum_j w0_j v_j
 // - x; w = w0 - Vb^T M (Vb w0 - [1; x]) (Vb w0 = [1; x + r]). L = (1/B)
 // sum_b sum_j (w - w*)^2 + lambda (1/B) sum_b |r|^2 / (3 s^2). dL/dw0 = Pi g
 // + (2 lambda / (3 B s^2)) (r . v_j) with g = 2 (w - w*) / B and the
 // projector Pi = I - Vb^T M Vb; dz = dL/dw0 - mean (the sum in w0). dz is
-// written in fp32 and bf16; the loss terms (residual without lambda) are
-// added to loss[0..1].
-__global__ void k_field_loss(FieldLoss fl) {
-  const uint32_t row = blockIdx.x;
-  if (row >= fl.B) return;
-  __shared__ float red[6 * 32];
-  const float* z = fl.z + (size_t)row * fl.ldz;
-  const float* wt = fl.wt + (size_t)row * fl.ldw;
-  const float* x = fl.x + 3 * (size_t)row;
-  float s1[1] = {0.0f};
-  for (uint32_t j = threadIdx.x; j < fl.V; j += blockDim.x) s1[0] += z[j];
-  block_sums<1>(s1, red);
-  const float add = (1.0f - s1[0]) / (float)fl.V;
-  float s3[3] = {0.0f, 0.0f, 0.0f};
-  for (uint32_t j = threadIdx.x; j < fl.V; j += blockDim.x) {
-    const float w0 = z[j] + add;
-    const float4 v = fl.verts[j];
-    s3[0] += w0 * v.x;
-    s3[1] += w0 * v.y;
-    s3[2] += w0 * v.z;
-  }
-  block_sums<3>(s3, red);
-  const float r[3] = {s3[0] - x[0], s3[1] - x[1], s3[2] - x[2]};
-  float u[4];
-  lp_correction(fl.M, r, u);
-  const float inv_b = 1.0f / (float)fl.B;
-  // pass: squared error of w and Vb g (g = 2 e / B)
-  float s5[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-  for (uint32_t j = threadIdx.x; j < fl.V; j += blockDim.x) {
-    const float4 v = fl.verts[j];
-    const float w = z[j] + add - (u[0] + (v.x * u[1] + v.y * u[2] + v.z * u[3]));
-    const float e = w - wt[j];
-    const float g = 2.0f * e * inv_b;
-    s5[0] += e * e;
-    s5[1] += g;
-    s5[2] += g * v.x;
-    s5[3] += g * v.y;
-    s5[4] += g * v.z;
-  }
-  block_sums<5>(s5, red);
-  float q[4];
+// written in fp32 (for the bias gradient) and in bf16, row by row and
+// transposed; the loss terms (residual without lambda) are added to
+// loss[0..1]. One warp per row, its outputs and targets in registers (lane l
+// holds columns l + 32 k), so the row's five sums take shuffles and no block
+// barrier; a block's kLossRows rows are transposed through shared memory.
+// OWN: columns per lane.
+template <int OWN>
+__global__ void __launch_bounds__(32 * kLossRows, 1) k_field_loss(FieldLoss fl) {
+  extern __shared__ __align__(16) unsigned char loss_smem[];
+  float4* sv = reinterpret_cast<float4*>(loss_smem);                // [V]
+  __nv_bfloat16* st = reinterpret_cast<__nv_bfloat16*>(sv + fl.V);   // [V][kLossRows]
+  __shared__ float s_loss[2][kLossRows];
+  const uint32_t V = fl.V, row0 = blockIdx.x * kLossRows;
+  const uint32_t lane = threadIdx.x & 31u, q = threadIdx.x >> 5, row = row0 + q;
+  for (uint32_t j = threadIdx.x; j < V; j += 32 * kLossRows) sv[j] = fl.verts[j];
+  const bool on = row < fl.B;
+  const float* z = fl.z + (size_t)(on ? row : 0u) * fl.ldz;
+  const float* wt = fl.target + (size_t)(on ? fl.idx[row] : 0u) * V;
+  float zr[OWN], tr[OWN];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
-    q[a] = fl.M[4 * a] * s5[1] + fl.M[4 * a + 1] * s5[2] + fl.M[4 * a + 2] * s5[3] +
-           fl.M[4 * a + 3] * s5[4];
-  const float cres = fl.lambda * 2.0f / (3.0f * (float)fl.B * fl.s2);
-  auto grad_w0 = [&](uint32_t j) {
-    const float4 v = fl.verts[j];
-    const float w = z[j] + add - (u[0] + (v.x * u[1] + v.y * u[2] + v.z * u[3]));
-    const float g = 2.0f * (w - wt[j]) * inv_b;
-    return g - (q[0] + (v.x * q[1] + v.y * q[2] + v.z * q[3])) +
-           cres * ((r[0] * v.x + r[1] * v.y) + r[2] * v.z);
-  };
-  float sg[1] = {0.0f};
-  for (uint32_t j = threadIdx.x; j < fl.V; j += blockDim.x) sg[0] += grad_w0(j);
-  block_sums<1>(sg, red);
-  const float gmean = sg[0] / (float)fl.V;
-  for (uint32_t j = threadIdx.x; j < fl.V; j += blockDim.x) {
-    const float dz = grad_w0(j) - gmean;
-    fl.dz[(size_t)row * fl.ldz + j] = dz;
-    fl.dzb[(size_t)row * fl.ldz + j] = __float2bfloat16_rn(dz);
+  for (int k = 0; k < OWN; ++k) {
+    const uint32_t j = lane + 32u * k;
+    zr[k] = j < V ? z[j] : 0.0f;
+    tr[k] = j < V ? wt[j] : 0.0f;
   }
-  if (threadIdx.x == 0) {
-    atomicAdd(&fl.loss[0], s5[0] * inv_b);
-    atomicAdd(&fl.loss[1], ((r[0] * r[0] + r[1] * r[1]) + r[2] * r[2]) /
-                               (3.0f * (float)fl.B * fl.s2));
+  __syncthreads();
+  if (on) {
+    const float* x = fl.x + 3 * (size_t)row;
+    const float inv_b = 1.0f / (float)fl.B;
+    float s1[1][4] = {}, t1[1];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k)
+      if (lane + 32u * k < V) s1[0][k & 3] += zr[k];
+    row_sums<1>(s1, t1);
+    const float add = (1.0f - t1[0]) / (float)V;
+    float s3[3][4] = {}, t3[3];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      const uint32_t j = lane + 32u * k;
+      if (j >= V) continue;
+      const float w0 = zr[k] + add;
+      const float4 v = sv[j];
+      s3[0][k & 3] += w0 * v.x;
+      s3[1][k & 3] += w0 * v.y;
+      s3[2][k & 3] += w0 * v.z;
+    }
+    row_sums<3>(s3, t3);
+    const float r[3] = {t3[0] - x[0], t3[1] - x[1], t3[2] - x[2]};
+    float u[4];
+    lp_correction(fl.M, r, u);
+    // squared error of w and Vb g (g = 2 e / B)
+    float s5[5][4] = {}, t5[5];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      const uint32_t j = lane + 32u * k;
+      if (j >= V) continue;
+      const float4 v = sv[j];
+      const float w = zr[k] + add - (u[0] + (v.x * u[1] + v.y * u[2] + v.z * u[3]));
+      const float e = w - tr[k];
+      const float g = 2.0f * e * inv_b;
+      s5[0][k & 3] += e * e;
+      s5[1][k & 3] += g;
+      s5[2][k & 3] += g * v.x;
+      s5[3][k & 3] += g * v.y;
+      s5[4][k & 3] += g * v.z;
+    }
+    row_sums<5>(s5, t5);
+    float qv[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      qv[a] = fl.M[4 * a] * t5[1] + fl.M[4 * a + 1] * t5[2] + fl.M[4 * a + 2] * t5[3] +
+              fl.M[4 * a + 3] * t5[4];
+    const float cres = fl.lambda * 2.0f / (3.0f * (float)fl.B * fl.s2);
+    float sg[1][4] = {}, tg[1];
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      const uint32_t j = lane + 32u * k;
+      if (j >= V) continue;
+      const float4 v = sv[j];
+      const float w = zr[k] + add - (u[0] + (v.x * u[1] + v.y * u[2] + v.z * u[3]));
+      const float g = 2.0f * (w - tr[k]) * inv_b;
+      tr[k] = g - (qv[0] + (v.x * qv[1] + v.y * qv[2] + v.z * qv[3])) +
+              cres * ((r[0] * v.x + r[1] * v.y) + r[2] * v.z);
+      sg[0][k & 3] += tr[k];
+    }
+    row_sums<1>(sg, tg);
+    const float gmean = tg[0] / (float)V;
+#pragma unroll
+    for (int k = 0; k < OWN; ++k) {
+      const uint32_t j = lane + 32u * k;
+      if (j >= V) continue;
+      const float dz = tr[k] - gmean;
+      const __nv_bfloat16 b = __float2bfloat16_rn(dz);
+      fl.dz[(size_t)row * fl.ldz + j] = dz;
+      fl.dzb[(size_t)row * fl.ldz + j] = b;
+      st[j * kLossRows + q] = b;
+    }
+    if (lane == 0) {
+      s_loss[0][q] = t5[0] * inv_b;
+      s_loss[1][q] = ((r[0] * r[0] + r[1] * r[1]) + r[2] * r[2]) / (3.0f * (float)fl.B * fl.s2);
+    }
+  } else if (lane == 0) {
+    s_loss[0][q] = s_loss[1][q] = 0.0f;
+  }
+  __syncthreads();
+  // one atomic per block and term (per row, the two words took most of 30 us)
+  if (threadIdx.x < 2) {
+    float t = 0.0f;
+    for (uint32_t k = 0; k < kLossRows; ++k) t += s_loss[threadIdx.x][k];
+    atomicAdd(&fl.loss[threadIdx.x], t);
+  }
+  // two rows of one output per 4-byte store (B and row0 are even)
+  const uint32_t rows = min(kLossRows, fl.B - row0);
+  for (uint32_t k = threadIdx.x; k < V * (kLossRows / 2); k += 32 * kLossRows) {
+    const uint32_t j = k / (kLossRows / 2), p = 2 * (k % (kLossRows / 2));
+    if (p < rows)
+      *reinterpret_cast<__nv_bfloat162*>(fl.dzT + (size_t)j * fl.B + row0 + p) =
+          *reinterpret_cast<const __nv_bfloat162*>(st + j * kLossRows + p);
   }
 }
 
-// dpre = dA * silu'(pre) (fp32 and bf16 copies), elementwise.
-__global__ void k_silu_back(uint32_t n, const float* __restrict__ da,
-                            const float* __restrict__ pre, float* __restrict__ dpre,
-                            __nv_bfloat16* __restrict__ dpreb) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float v = da[i] * silu_grad(pre[i]);
-  dpre[i] = v;
-  dpreb[i] = __float2bfloat16_rn(v);
-}
-
-// Column sums of g [B x ld] over rows -> out [N] (bias gradients).
-__global__ void k_colsum(const float* __restrict__ g, uint32_t B, uint32_t N, uint32_t ld,
-                         float* __restrict__ out) {
-  const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= N) return;
-  float s = 0.0f;
-  for (uint32_t r = 0; r < B; ++r) s += g[(size_t)r * ld + c];
-  out[c] = s;
-}
-
-// Adam (Kingma & Ba 2015) on fp32 master weights, refreshing the bf16 copy:
-// m = b1 m + (1-b1) g; v = b2 v + (1-b2) g^2; p -= lr mh / (sqrt(vh) + eps)
-// with the bias corrections mh = m c1, vh = v c2.
-__global__ void k_adam(uint32_t n, float* __restrict__ p, const float* __restrict__ g,
-                       float* __restrict__ m, float* __restrict__ v,
-                       __nv_bfloat16* __restrict__ pb, float lr, float b1, float b2, float eps,
-                       float c1, float c2) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.0f - b1) * gi;
-  const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  p[i] = pi;
-  if (pb) pb[i] = __float2bfloat16_rn(pi);
+// Gradients and Adam (Kingma & Ba 2015) on the fp32 master weights, one
+// parameter per thread: g = the splits' partial sums in split order (weights)
+// or the column sum (biases, in g already); m = b1 m + (1-b1) g; v = b2 v +
+// (1-b2) g^2; p -= lr mh / (sqrt(vh) + eps) with the bias corrections mh = m
+// c1, vh = v c2; refreshes the bf16 copy and the transposed weights.
+__global__ void __launch_bounds__(256) k_field_update(FieldUpdate a) {
+  const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= a.off[10]) return;
+  float gi = 0.0f;
+  bool weight = false;
+#pragma unroll
+  for (int l = 0; l < 5; ++l) {
+    const uint32_t o = a.off[2 * l];
+    const uint32_t n = l == 4 ? a.V * kHid : (uint32_t)kHid * (l == 0 ? kIn : kHid);
+    if (i < o || i - o >= n) continue;
+    weight = true;
+    if (a.splits == 16) {
+#pragma unroll
+      for (uint32_t z = 0; z < 16; ++z) gi += a.ws[l][(size_t)z * n + (i - o)];
+    } else {
+      for (uint32_t z = 0; z < a.splits; ++z) gi += a.ws[l][(size_t)z * n + (i - o)];
+    }
+  }
+  if (weight)
+    a.g[i] = gi;
+  else
+    gi = a.g[i];
+  if (!a.adam) return;
+  const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * gi;
+  const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * gi * gi;
+  a.m[i] = mi;
+  a.v[i] = vi;
+  const float pi = a.p[i] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);
+  a.p[i] = pi;
+  const __nv_bfloat16 w = __float2bfloat16_rn(pi);
+  a.pb[i] = w;
+  put_transposed(a.off, a.ldV, a.wT, i, w);
 }
 
 // ---- frame: per-frame projection and fused inference ---------------------------
@@ -585,51 +678,43 @@ __global__ void __launch_bounds__(kApWarps * 32, 1) k_field_apply(FieldInfer fi)
 
 cudaError_t launch_field_gather(const FieldBatch& b, cudaStream_t s) {
   if (b.B == 0) return cudaSuccess;
-  k_field_gather<<<b.B, 128, 0, s>>>(b);
+  k_field_gather<<<(b.B + kGatherRows - 1) / kGatherRows, 256, 0, s>>>(b);
   return cudaGetLastError();
 }
 
-cudaError_t launch_transpose_f32(const float* in, uint32_t R, uint32_t C, uint32_t ldi,
-                                 __nv_bfloat16* out, uint32_t ldo, cudaStream_t s) {
-  if (R == 0 || C == 0) return cudaSuccess;
-  k_transpose<float><<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(in, R, C, ldi, out,
-                                                                                ldo);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_transpose_bf16(const __nv_bfloat16* in, uint32_t R, uint32_t C, uint32_t ldi,
-                                  __nv_bfloat16* out, uint32_t ldo, cudaStream_t s) {
-  if (R == 0 || C == 0) return cudaSuccess;
-  k_transpose<__nv_bfloat16><<<dim3((C + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(
-      in, R, C, ldi, out, ldo);
+cudaError_t launch_field_refresh(const uint32_t* off, uint32_t V, uint32_t ldV, const float* p,
+                                 __nv_bfloat16* pb, __nv_bfloat16* const* wT, cudaStream_t s) {
+  RefreshArgs a{};
+  for (int k = 0; k < 11; ++k) a.off[k] = off[k];
+  a.V = V;
+  a.ldV = ldV;
+  a.p = p;
+  a.pb = pb;
+  for (int l = 0; l < 4; ++l) a.wT[l] = wT ? wT[l] : nullptr;
+  k_field_refresh<<<(off[10] + 255) / 256, 256, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s) {
   if (l.B == 0) return cudaSuccess;
-  k_field_loss<<<l.B, 128, 0, s>>>(l);
-  return cudaGetLastError();
+  if (l.V > 1024u || (l.B & 1u)) return cudaErrorInvalidValue;
+  const size_t smem = (size_t)l.V * (16 + 2 * kLossRows);
+  auto run = [&](auto kernel) {
+    if (smem > 48 * 1024) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    kernel<<<(l.B + kLossRows - 1) / kLossRows, 32 * kLossRows, smem, s>>>(l);
+    return cudaGetLastError();
+  };
+  if (l.V <= 192u) return run(k_field_loss<6>);
+  if (l.V <= 672u) return run(k_field_loss<21>);
+  return run(k_field_loss<32>);
 }
 
-cudaError_t launch_silu_back(uint32_t n, const float* da, const float* pre, float* dpre,
-                             __nv_bfloat16* dpreb, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  k_silu_back<<<(n + 255) / 256, 256, 0, s>>>(n, da, pre, dpre, dpreb);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_colsum(const float* g, uint32_t B, uint32_t N, uint32_t ld, float* out,
-                          cudaStream_t s) {
-  if (N == 0) return cudaSuccess;
-  k_colsum<<<(N + 127) / 128, 128, 0, s>>>(g, B, N, ld, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_adam(uint32_t n, float* p, const float* g, float* m, float* v,
-                        __nv_bfloat16* pb, float lr, float b1, float b2, float eps, float c1,
-                        float c2, cudaStream_t s) {
-  if (n == 0) return cudaSuccess;
-  k_adam<<<(n + 255) / 256, 256, 0, s>>>(n, p, g, m, v, pb, lr, b1, b2, eps, c1, c2);
+cudaError_t launch_field_update(const FieldUpdate& u, cudaStream_t s) {
+  k_field_update<<<(u.off[10] + 255) / 256, 256, 0, s>>>(u);
   return cudaGetLastError();
 }
 

@@ -164,6 +164,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+        "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
@@ -505,18 +514,25 @@ __global__ void __launch_bounds__(kTcWG * 128, 1) k_field_infer_tc(FieldInfer fi
 }
 
 // ---- training GEMMs: C = A B^T (+ bias), D = bf16(silu(C)) -------------------
-// One CTA of 128 threads per 128 x 128 output tile. K is consumed in 64-wide
-// blocks through a 4-stage ring: every thread copies its share of a block's
-// A and B rows into shared memory with 16-byte cp.async (rows past M or N and
-// columns past K zero-filled) in the K-major 128-byte-swizzle layout, one
-// elected thread issues the block's four K = 16 tcgen05 MMAs into a 128-column
-// TMEM accumulator and commits them to the stage's mbarrier, and the copies
-// run two blocks ahead of the MMAs; a stage is refilled once the MMAs that
-// read it have completed. The epilogue reads the accumulator row by row
-// (TMEM lane = output row) and applies the bias and SiLU.
-constexpr uint32_t kGmTile = 128, kGmBK = 64, kGmStages = 4, kGmAhead = 2;
-constexpr uint32_t kGmStageBytes = 2 * kGmTile * kGmBK * 2;   // A and B, 32 KB
-constexpr uint32_t kGmSmem = kGmStages * kGmStageBytes + 256 + 1024;
+// One CTA of 256 threads per 128 x NT output tile. K is consumed in 64-wide
+// blocks through a ring of 2 A stages: every thread copies its share of a
+// block's A and B rows into shared memory with 16-byte cp.async (rows past M
+// or N and columns past K zero-filled) in the K-major 128-byte-swizzle layout,
+// one elected thread issues the block's four K = 16 tcgen05 MMAs into an
+// NT-column TMEM accumulator and commits them to the stage's mbarrier, and the
+// copies run A blocks ahead of the MMAs; a stage is refilled once the MMAs
+// that read it have completed. The epilogue reads the accumulator row by row
+// (TMEM lane = output row), each warpgroup half of the columns. The products
+// are small (4,096 x 128 x 128), so the epilogue's instructions bound them: NT
+// = 32 puts 128 CTAs on a layer instead of 32 (16 us a layer with NT = 128).
+constexpr uint32_t kGmTile = 128, kGmBK = 64;
+constexpr int kGmThreads = 256;
+constexpr uint32_t kGmSumRows = 64, kGmSumStages = 8;  // column-sum ring
+__host__ __device__ constexpr uint32_t gm_stage_bytes(uint32_t nt) { return (kGmTile + nt) * kGmBK * 2; }
+// dynamic shared memory of `stages` stages, rounded so that the barriers follow
+__host__ __device__ constexpr uint32_t gm_smem(uint32_t nt, uint32_t stages) {
+  return stages * gm_stage_bytes(nt) + 256 + 1024;
+}
 
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes)
@@ -532,36 +548,28 @@ __device__ __forceinline__ void cp_async_wait() {
 
 constexpr uint32_t kGmMaxSplits = 16;
 
-// C[r][c] = sum over splits z (in order) of ws[z][r][c].
-__global__ void k_split_reduce(const float* __restrict__ ws, uint32_t splits, uint32_t M,
-                               uint32_t N, float* __restrict__ C, uint32_t ldc) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * N) return;
-  float acc = 0.0f;
-  for (uint32_t z = 0; z < splits; ++z) acc += ws[(size_t)z * M * N + i];
-  C[(size_t)(i / N) * ldc + i % N] = acc;
-}
-
-template <int EPI>
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
+// One 128 x NT tile: rows m0.., columns n0.., K blocks [kb0, kb0 + nk).
+template <int EPI, int NT, uint32_t A>
+__device__ __forceinline__ void gemm_tile(const GemmArgs& g, uint32_t m0, uint32_t n0, uint32_t z,
+                                          uint32_t splits) {
   extern __shared__ unsigned char gm_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(gm_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* s_bar = reinterpret_cast<uint64_t*>(sm + kGmStages * kGmStageBytes);  // [stages]
-  uint32_t* s_tmem = reinterpret_cast<uint32_t*>(s_bar + kGmStages);
-  volatile uint32_t* s_ok = s_tmem + 1;  // [2], alternating by block
+  constexpr uint32_t kStageBytes = gm_stage_bytes(NT), kStages = 2 * A;
+  __shared__ __align__(8) uint64_t s_bar[kStages];
+  __shared__ uint32_t s_words[4];
+  uint32_t* s_tmem = s_words;
+  volatile uint32_t* s_ok = s_words + 1;  // [2], alternating by block
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t m0 = blockIdx.y * kGmTile, n0 = blockIdx.x * kGmTile;
   // split z of K: blocks [kb0, kb0 + nk) of the K range
-  const uint32_t nkb = (g.K + kGmBK - 1) / kGmBK, per = (nkb + gridDim.z - 1) / gridDim.z;
-  const uint32_t kb0 = min(nkb, blockIdx.z * per), nk = min(nkb, kb0 + per) - kb0;
-  const bool split = gridDim.z > 1;
-  if (tid < (int)kGmStages)
+  const uint32_t nkb = (g.K + kGmBK - 1) / kGmBK, per = (nkb + splits - 1) / splits;
+  const uint32_t kb0 = min(nkb, z * per), nk = min(nkb, kb0 + per) - kb0;
+  if (tid < (int)kStages)
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&s_bar[tid])));
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
                      smem_u32(s_tmem)),
-                 "r"(kGmTile));
+                 "r"((uint32_t)NT));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
   }
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -570,13 +578,13 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
   tc_fence_after();
   const uint32_t tmem = *s_tmem;
   const uint32_t base = smem_u32(sm);
-  const uint32_t idesc = idesc_bf16(kGmTile, kGmTile, 0, 0);
+  const uint32_t idesc = idesc_bf16(kGmTile, NT, 0, 0);
 
   // block kb of A rows m0.. and B rows n0.. into stage kb % stages
   auto load = [&](uint32_t kb) {
-    const uint32_t st = base + (kb % kGmStages) * kGmStageBytes, k0 = (kb0 + kb) * kGmBK;
+    const uint32_t st = base + (kb % kStages) * kStageBytes, k0 = (kb0 + kb) * kGmBK;
 #pragma unroll 4
-    for (uint32_t c = (uint32_t)tid; c < 2 * kGmTile * 8; c += 128) {
+    for (uint32_t c = (uint32_t)tid; c < (kGmTile + NT) * 8; c += kGmThreads) {
       const bool isb = c >= kGmTile * 8;
       const uint32_t cc = isb ? c - kGmTile * 8 : c, row = cc >> 3, ch = cc & 7;
       const uint32_t grow = (isb ? n0 : m0) + row, R = isb ? g.N : g.M, k = k0 + ch * 8;
@@ -593,36 +601,36 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
     }
   };
 #pragma unroll
-  for (uint32_t p = 0; p < kGmAhead; ++p) {
+  for (uint32_t p = 0; p < A; ++p) {
     if (p < nk) load(p);
     cp_async_commit();
   }
   bool ok = true;
   uint32_t issued = 0;  // blocks whose MMAs were issued (block-uniform)
   for (uint32_t kb = 0; kb < nk; ++kb) {
-    cp_async_wait<kGmAhead - 1>();  // this thread's copies of block kb have landed
+    cp_async_wait<A - 1>();  // this thread's copies of block kb have landed
     fence_async_smem();
     // the stage refilled below was read by the MMAs of block kb - ahead
-    if (tid == 0 && kb >= kGmAhead) {
-      const uint32_t q = kb - kGmAhead;
-      s_ok[kb & 1u] = mbar_wait(smem_u32(&s_bar[q % kGmStages]), (q / kGmStages) & 1u) ? 1u : 0u;
+    if (tid == 0 && kb >= A) {
+      const uint32_t q = kb - A;
+      s_ok[kb & 1u] = mbar_wait(smem_u32(&s_bar[q % kStages]), (q / kStages) & 1u) ? 1u : 0u;
     }
     __syncthreads();
-    if (kb >= kGmAhead && s_ok[kb & 1u] == 0u) {
+    if (kb >= A && s_ok[kb & 1u] == 0u) {
       ok = false;
       break;
     }
     if (tid == 0) {
       tc_fence_after();
-      const uint32_t a = base + (kb % kGmStages) * kGmStageBytes, b = a + kGmTile * 128;
+      const uint32_t a = base + (kb % kStages) * kStageBytes, b = a + kGmTile * 128;
 #pragma unroll
       for (uint32_t k16 = 0; k16 < kGmBK / 16; ++k16)
         mma_bf16_tc(tmem, sw128_desc(a + k16 * 32), sw128_desc(b + k16 * 32), idesc,
                     (kb > 0 || k16 > 0) ? 1u : 0u);
-      mma_commit(smem_u32(&s_bar[kb % kGmStages]));
+      mma_commit(smem_u32(&s_bar[kb % kStages]));
     }
     issued = kb + 1;
-    if (kb + kGmAhead < nk) load(kb + kGmAhead);
+    if (kb + A < nk) load(kb + A);
     cp_async_commit();
   }
   cp_async_wait<0>();
@@ -631,7 +639,7 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
     bool done = true;
     if (issued > 0) {
       const uint32_t q = issued - 1;
-      done = mbar_wait(smem_u32(&s_bar[q % kGmStages]), (q / kGmStages) & 1u);
+      done = mbar_wait(smem_u32(&s_bar[q % kStages]), (q / kStages) & 1u);
     }
     s_ok[0] = (ok && done) ? 1u : 0u;
     if ((!ok || !done) && g.status) {
@@ -644,63 +652,80 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
   ok = s_ok[0] != 0u;
   tc_fence_after();
   if (ok) {
-    const uint32_t row = m0 + 32u * (uint32_t)warp + (uint32_t)lane;
-    const uint32_t t_row = tmem + ((uint32_t)warp * 32u << 16);
-    const bool vec_c = ((g.ldc & 3u) == 0u) && (((uintptr_t)g.C & 15u) == 0u);
+    const uint32_t wr = (uint32_t)warp & 3u;  // the TMEM lanes a warp may read
+    const uint32_t row = m0 + 32u * wr + (uint32_t)lane;
+    const uint32_t t_row = tmem + (wr * 32u << 16);
+    const bool in = row < g.M;
+    float* C = EPI == kEpiSplit ? g.C + (size_t)z * g.M * g.N : g.C;
+    const uint32_t ldc = EPI == kEpiSplit ? g.N : g.ldc;
+    const bool vec_c = ((ldc & 3u) == 0u) && (((uintptr_t)C & 15u) == 0u);
     const bool vec_d = ((g.ldd & 7u) == 0u) && (((uintptr_t)g.D & 15u) == 0u);
-#pragma unroll 1
-    for (uint32_t c0 = 0; c0 < kGmTile; c0 += 32) {
-      uint32_t v[32];
-      if (nk > 0) {
-        tmem_ld32_nowait<0>(t_row + c0, v);  // every lane of the warp loads (aligned)
-        tmem_wait_ld();
-      } else {
+    constexpr int W = NT / 2;  // this warpgroup's columns
+    const uint32_t c0 = ((uint32_t)warp >> 2) * W, col0 = n0 + c0;
+    uint32_t v[W];
+    if (nk > 0) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0u;
-      }
-      const uint32_t col0 = n0 + c0;
-      if (row >= g.M || col0 >= g.N) continue;
-      float x[32];
+      for (int q = 0; q < W; q += 16) tmem_ld16_nowait(t_row + c0 + q, v + q);  // aligned
+      tmem_wait_ld();
+    } else {
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
+      for (int i = 0; i < W; ++i) v[i] = 0u;
+    }
+    if (col0 < g.N && in) {
+      const bool whole = col0 + W <= g.N;
+      float x[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
         x[i] = __uint_as_float(v[i]);
-        if (EPI != kEpiF32 && col0 + i < g.N) x[i] += g.bias[col0 + i];
+        if ((EPI == kEpiBias || EPI == kEpiBiasSilu) && col0 + i < g.N) x[i] += g.bias[col0 + i];
       }
-      // a split's partial sums go to its slice of the workspace ([M][N] each)
-      float* crow = split ? g.ws + ((size_t)blockIdx.z * g.M + row) * g.N + col0
-                          : g.C + (size_t)row * g.ldc + col0;
-      if (split) {
+      if (EPI == kEpiBack) {
+        const float* prow = g.pre + (size_t)row * ldc + col0;  // N is a multiple of W
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (col0 + i < g.N) crow[i] = x[i];
-        continue;
+        for (int i = 0; i < W; i += 4) {
+          const float4 p4 = *reinterpret_cast<const float4*>(prow + i);
+          const float p[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float sg = 1.0f / (1.0f + __expf(-p[e]));
+            x[i + e] = x[i + e] * (sg * (1.0f + p[e] * (1.0f - sg)));
+          }
+        }
       }
-      if (vec_c && col0 + 32 <= g.N) {
+      float* crow = C + (size_t)row * ldc + col0;
+      if (vec_c && whole) {
 #pragma unroll
-        for (int i = 0; i < 32; i += 4)
+        for (int i = 0; i < W; i += 4)
           *reinterpret_cast<float4*>(crow + i) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
       } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
+        for (int i = 0; i < W; ++i)
           if (col0 + i < g.N) crow[i] = x[i];
       }
-      if (EPI == kEpiBiasSilu) {
-        __nv_bfloat16* drow = g.D + (size_t)row * g.ldd + col0;
-        if (vec_d && col0 + 32 <= g.N) {
+      if (EPI == kEpiBiasSilu || EPI == kEpiBack) {
+        if (EPI == kEpiBiasSilu) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint32_t w[4];
+          for (int i = 0; i < W; ++i) x[i] = x[i] * (1.0f / (1.0f + __expf(-x[i])));
+        }
+        if (g.D) {
+          __nv_bfloat16* drow = g.D + (size_t)row * g.ldd + col0;
+          if (vec_d && whole) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float a0 = x[i + 2 * e], a1 = x[i + 2 * e + 1];
-              w[e] = pack2(a0 * (1.0f / (1.0f + __expf(-a0))), a1 * (1.0f / (1.0f + __expf(-a1))));
-            }
-            *reinterpret_cast<uint4*>(drow + i) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int i = 0; i < W; i += 8)
+              *reinterpret_cast<uint4*>(drow + i) =
+                  make_uint4(pack2(x[i], x[i + 1]), pack2(x[i + 2], x[i + 3]),
+                             pack2(x[i + 4], x[i + 5]), pack2(x[i + 6], x[i + 7]));
+          } else {
+#pragma unroll
+            for (int i = 0; i < W; ++i)
+              if (col0 + i < g.N) drow[i] = __float2bfloat16_rn(x[i]);
           }
-        } else {
+        }
+        if (g.DT) {
+          // a column of the tile is 32 consecutive rows of the transpose
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (col0 + i < g.N) drow[i] = __float2bfloat16_rn(x[i] * (1.0f / (1.0f + __expf(-x[i]))));
+          for (int i = 0; i < W; ++i)
+            if (col0 + i < g.N) g.DT[(size_t)(col0 + i) * g.ldt + row] = __float2bfloat16_rn(x[i]);
         }
       }
     }
@@ -710,7 +735,80 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmArgs g) {
   tc_fence_after();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem),
-                 "r"(kGmTile));
+                 "r"((uint32_t)NT));
+}
+
+template <int EPI, int NT, uint32_t A>
+__global__ void __launch_bounds__(kGmThreads) k_gemm_tc(GemmArgs g) {
+  gemm_tile<EPI, NT, A>(g, blockIdx.y * kGmTile, blockIdx.x * NT, 0, 1);
+}
+
+// Column sums over the rows of in [B][ld], 32 columns per block, each column's
+// rows added one after the other in row order: the ring of 64-row stages is
+// filled by the whole block with cp.async while warp 0 adds (4 cycles a row;
+// one thread per column that walked the rows in memory took 160 us at 4,096
+// rows).
+__device__ __forceinline__ void column_sums(const float* in, uint32_t B, uint32_t N, uint32_t ld,
+                                            uint32_t c0, float* out) {
+  extern __shared__ unsigned char gm_raw[];
+  float* ring = reinterpret_cast<float*>(gm_raw);  // [kGmSumStages][kGmSumRows][32]
+  const uint32_t tid = threadIdx.x;
+  const uint32_t stages = (B + kGmSumRows - 1) / kGmSumRows;
+  auto load = [&](uint32_t s) {
+    const uint32_t st = smem_u32(ring) + (s % kGmSumStages) * kGmSumRows * 128;
+#pragma unroll
+    for (uint32_t c = tid; c < kGmSumRows * 8; c += kGmThreads) {
+      const uint32_t r = s * kGmSumRows + (c >> 3), col = c0 + (c & 7) * 4;
+      const bool ok = s < stages && r < B && col < ld;
+      cp_async16_zfill(st + c * 16, ok ? in + (size_t)r * ld + col : in, ok ? 16u : 0u);
+    }
+    cp_async_commit();
+  };
+  for (uint32_t s = 0; s + 1 < kGmSumStages; ++s) load(s);
+  float acc = 0.0f;
+  for (uint32_t s = 0; s < stages; ++s) {
+    cp_async_wait<(int)kGmSumStages - 2>();
+    __syncthreads();  // stage s has landed for every thread; stage s - 1 has been read
+    load(s + kGmSumStages - 1);
+    if (tid < 32) {
+      const float* p = ring + (s % kGmSumStages) * kGmSumRows * 32 + tid;
+      const uint32_t rows = min(kGmSumRows, B - s * kGmSumRows);
+      if (rows == kGmSumRows) {
+#pragma unroll
+        for (uint32_t r = 0; r < kGmSumRows; ++r) acc += p[r * 32];
+      } else {
+        for (uint32_t r = 0; r < rows; ++r) acc += p[r * 32];
+      }
+    }
+  }
+  cp_async_wait<0>();
+  if (tid < 32 && c0 + tid < N) out[c0 + tid] = acc;
+}
+
+// Every layer's weight and bias gradients (K = the batch) in one launch: the
+// first blocks take 32 bias columns each, the others a tile and a K range of
+// a weight gradient, over the whole chip instead of 1 to 6 tiles per launch;
+// the ranges' partial sums are added in order by the update kernel.
+__global__ void __launch_bounds__(kGmThreads) k_gemm_grads(GemmBatch b, uint32_t sum_blocks) {
+  uint32_t i = blockIdx.x;
+  if (i < sum_blocks) {
+#pragma unroll 1
+    for (int p = 0; p < kGradProblems; ++p) {
+      const uint32_t nb = (b.sum_n[p] + 31) / 32;
+      if (i < nb) {
+        column_sums(b.sum[p], b.g[p].K, b.sum_n[p], b.sum_ld[p], 32 * i, b.sum_out[p]);
+        return;
+      }
+      i -= nb;
+    }
+    return;
+  }
+  i -= sum_blocks;
+  const uint32_t z = i / b.first[kGradProblems], t = i % b.first[kGradProblems];
+  uint32_t p = 0;
+  while (p + 1 < (uint32_t)kGradProblems && t >= b.first[p + 1]) ++p;
+  const uint32_t nt = (b.g[p].N + 63) / 64, q = t - b.first[p];
+  gemm_tile<kEpiSplit, 64, 1>(b.g[p], q / nt * kGmTile, q % nt * 64, z, b.splits);
 }
 
 }  // namespace
@@ -743,44 +841,46 @@ cudaError_t launch_gemm_nt(const GemmArgs& g, int epi, cudaStream_t s) {
   if (g.M == 0 || g.N == 0) return cudaSuccess;
   if ((g.lda & 7) || (g.ldb & 7)) return cudaErrorInvalidValue;
   if (((uintptr_t)g.A & 15) || ((uintptr_t)g.B & 15)) return cudaErrorInvalidValue;
-  static int sm_count = 0;
-  if (sm_count == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      sm_count = 148;
+  // up to 2 A stages, as many as there are K blocks
+  auto run = [&](auto kernel, uint32_t nt, uint32_t A) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)gm_smem(nt, 2 * A));
+    if (e != cudaSuccess) return e;
+    const uint32_t stages = std::min((g.K + kGmBK - 1) / kGmBK, 2 * A);
+    const dim3 grid((g.N + nt - 1) / nt, (g.M + kGmTile - 1) / kGmTile);
+    kernel<<<grid, kGmThreads, gm_smem(nt, stages), s>>>(g);
+    return cudaGetLastError();
+  };
+  if (epi == kEpiBias) return run(k_gemm_tc<kEpiBias, 64, 2>, 64, 2);
+  if (epi == kEpiBiasSilu) return run(k_gemm_tc<kEpiBiasSilu, 32, 2>, 32, 2);
+  if (epi == kEpiBack && g.N % 16 == 0 && g.ldc % 4 == 0) {
+    // the output layer's K is the cage's vertices: four blocks in flight
+    if (g.K > 4 * kGmBK) return run(k_gemm_tc<kEpiBack, 32, 4>, 32, 4);
+    return run(k_gemm_tc<kEpiBack, 32, 2>, 32, 2);
   }
-  dim3 grid((g.N + kGmTile - 1) / kGmTile, (g.M + kGmTile - 1) / kGmTile, 1);
-  // Long K over few tiles (the weight gradients: K = the batch): split K so
-  // that the grid covers the SMs; the partial sums are added in split order
-  // (deterministic) by k_split_reduce.
-  const uint32_t tiles = grid.x * grid.y, nkb = (g.K + kGmBK - 1) / kGmBK;
-  if (epi == kEpiF32 && g.ws && tiles * 2 <= (uint32_t)sm_count && nkb >= 8) {
-    uint32_t z = std::min<uint32_t>({(uint32_t)sm_count / tiles, nkb / 4, kGmMaxSplits});
-    while (z > 1 && (size_t)z * g.M * g.N > g.ws_floats) --z;
-    grid.z = std::max<uint32_t>(1, z);
+  return cudaErrorInvalidValue;
+}
+
+// K ranges of the weight gradients: at least four K blocks each, at most 16.
+uint32_t grad_splits(uint32_t B) {
+  const uint32_t nkb = (B + kGmBK - 1) / kGmBK;
+  return nkb >= 8 ? std::min(nkb / 4, kGmMaxSplits) : 1u;
+}
+
+cudaError_t launch_gemm_grads(const GemmBatch& b, cudaStream_t s) {
+  for (int p = 0; p < kGradProblems; ++p) {
+    const GemmArgs& g = b.g[p];
+    if ((g.lda & 7) || (g.ldb & 7) || (g.N & 15)) return cudaErrorInvalidValue;
+    if (((uintptr_t)g.A & 15) || ((uintptr_t)g.B & 15)) return cudaErrorInvalidValue;
   }
-  cudaError_t e;
-  if (epi == kEpiF32) {
-    e = cudaFuncSetAttribute(k_gemm_tc<kEpiF32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kGmSmem);
-    if (e == cudaSuccess) k_gemm_tc<kEpiF32><<<grid, 128, kGmSmem, s>>>(g);
-    if (e == cudaSuccess && grid.z > 1) {
-      e = cudaGetLastError();
-      const uint32_t n = g.M * g.N;
-      if (e == cudaSuccess)
-        k_split_reduce<<<(n + 255) / 256, 256, 0, s>>>(g.ws, grid.z, g.M, g.N, g.C, g.ldc);
-    }
-  } else if (epi == kEpiBias) {
-    e = cudaFuncSetAttribute(k_gemm_tc<kEpiBias>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kGmSmem);
-    if (e == cudaSuccess) k_gemm_tc<kEpiBias><<<grid, 128, kGmSmem, s>>>(g);
-  } else {
-    e = cudaFuncSetAttribute(k_gemm_tc<kEpiBiasSilu>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGmSmem);
-    if (e == cudaSuccess) k_gemm_tc<kEpiBiasSilu><<<grid, 128, kGmSmem, s>>>(g);
-  }
-  return e != cudaSuccess ? e : cudaGetLastError();
+  const uint32_t smem = std::max(gm_smem(64, 2), kGmSumStages * kGmSumRows * 128);
+  const cudaError_t e =
+      cudaFuncSetAttribute(k_gemm_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  uint32_t sums = 0;
+  for (int p = 0; p < kGradProblems; ++p) sums += (b.sum_n[p] + 31) / 32;
+  k_gemm_grads<<<sums + b.first[kGradProblems] * b.splits, kGmThreads, smem, s>>>(b, sums);
+  return cudaGetLastError();
 }
 
 }  // namespace cgs

@@ -1638,9 +1638,7 @@ int cgs_mvc_field_params(cgs_ctx* ctx, float* dst, const float* src) {
     field_changed(ctx);
     cudaStream_t s = ctx->stream;
     CGS_CUDA(cudaMemcpyAsync(f.p32.p, src, bytes, cudaMemcpyHostToDevice, s), "field params");
-    // bf16 copy: a 1 x total transpose is an elementwise conversion
-    CGS_CUDA(launch_transpose_f32(f.p32.as<float>(), 1, f.total(), f.total(),
-                                  f.pb.as<__nv_bfloat16>(), 1, s), "field params");
+    CGS_CUDA(f.refresh(s), "field params");
     CGS_CUDA(cudaMemsetAsync(f.m1.p, 0, bytes, s), "field params");
     CGS_CUDA(cudaMemsetAsync(f.m2.p, 0, bytes, s), "field params");
     CGS_CUDA(cudaStreamSynchronize(s), "field params");
@@ -1688,7 +1686,7 @@ int cgs_mvc_field_train(cgs_ctx* ctx, uint64_t n, const float* d_points, const f
                        lambda, s), "field forward");
     CGS_CUDA(f.backward(batch, s), "field backward");
     const double c = 0.5 * (1.0 + std::cos(3.141592653589793 * (double)t / (double)steps));
-    CGS_CUDA(f.adam(lr * (float)(0.05 + 0.95 * c), s), "field adam");
+    CGS_CUDA(f.update(batch, lr * (float)(0.05 + 0.95 * c), s), "field update");
   }
   float hl[2] = {0.0f, 0.0f};
   CGS_CUDA(cudaMemcpyAsync(hl, f.loss.p, 8, cudaMemcpyDeviceToHost, s), "field train");
@@ -1712,6 +1710,7 @@ int cgs_mvc_field_grads(cgs_ctx* ctx, uint64_t n, const float* d_points, const f
   CGS_CUDA(f.forward(d_points, d_weights, (uint32_t)n, (uint32_t)n, 0, ctx->mvc_rest.as<float4>(),
                      lambda, s), "field forward");
   CGS_CUDA(f.backward((uint32_t)n, s), "field backward");
+  CGS_CUDA(f.update((uint32_t)n, 0.0f, s), "field gradients");
   float hl[2];
   CGS_CUDA(cudaMemcpyAsync(hl, f.loss.p, 8, cudaMemcpyDeviceToHost, s), "field grads");
   CGS_TRY(field_status(ctx, "field gradients"));

@@ -2,33 +2,43 @@
 // render/kernels/compositor.rs:727-883) for 16x16 tiles (the reference's)
 // and 8x8 or 32x16 tiles (the autotuner's other shapes).
 //
-// One block per screen tile, one pixel per thread (64, 256 or 512 threads).
-// The tile's depth-sorted splat list is consumed in batches of 256: each
-// batch's 48-byte splat records are gathered from the Stage 2 record array
-// into shared memory by the whole block, three 16-byte cp.async copies per
-// record (measured faster than one cp.async.bulk per record completing on
-// an mbarrier: 6.5 vs 6.3 x 10^11 pixel-entry pairs/s on the 1080p frame),
-// double buffered so the next batch is in flight while the current one is
-// blended. Blending follows the reference: skip opacity <= 1/255; q = -(a dx^2 +
-// 2 b dx dy + c dy^2)/2 clamped to <= 0; skip q < -4; alpha = min(0.99,
-// op e^q); skip alpha < 1/255; front-to-back accumulate; a pixel stops at
-// T < 1e-3 (T := 0). The q cut and the alpha cut are evaluated exactly as the
-// host restatement does (IEEE-rounded q, the deterministic exp near the cut),
-// so the only differences are last-bit colour sums and the rare pixel whose
-// transmittance lands within an ulp of 1e-3 (bounded by that 1e-3). The block
-// stops when no pixel is still accumulating (the reference's double-buffered
-// tile_alive vote). Between batches the pixels that are still accumulating are
-// re-packed into the lowest threads of the block, so a warp whose 32 pixels
-// have all saturated stops issuing work instead of running the batch with
-// dead lanes. Output is RGBA8 packed in u32 rows padded to 64 pixels,
-// optionally also RGBA f32. A block never exits with a copy still in flight
-// into its shared memory.
+// One block per screen tile, one pixel per thread (64, 256 or 512 threads), a
+// warp per 8x4 pixels. The tile's depth-sorted splat list is consumed in
+// batches of 128: each batch's 48-byte splat records are gathered from the
+// Stage 2 record array into shared memory by the whole block, three 16-byte
+// cp.async copies per record (measured faster than one cp.async.bulk per
+// record completing on an mbarrier: 6.5 vs 6.3 x 10^11 pixel-entry pairs/s on
+// the 1080p frame), double buffered so the next batch is in flight while the
+// current one is blended. Blending follows the reference: skip opacity <=
+// 1/255; q = -(a dx^2 + 2 b dx dy + c dy^2)/2 clamped to <= 0; skip q < -4;
+// alpha = min(0.99, op e^q); skip alpha < 1/255; front-to-back accumulate; a
+// pixel stops at T < 1e-3 (T := 0). The q cut and the alpha cut are evaluated
+// exactly as the host restatement does (IEEE-rounded q, the deterministic exp
+// near the cut), so the only differences are last-bit colour sums and the rare
+// pixel whose transmittance lands within an ulp of 1e-3 (bounded by that
+// 1e-3).
+//
+// A tile's lists are walked warp by warp: when a batch has landed, each of its
+// entries is tested once against the warps' pixel blocks with the splat's
+// extents (a bound on where it can pass the cuts, with a margin for the
+// rounding of q), the ballots give every warp the entries that can touch it,
+// and the warp evaluates only those, four at a time without a branch: the four
+// opacities are independent, an entry that fails a cut blends with opacity 0
+// (which leaves the sums and T as they are, bit for bit, as does any entry
+// once T is 0), and only the transmittance is serial. One entry at a time, a
+// relevant entry took 300-400 cycles of dependent latency, and a frame waits
+// for its heaviest tiles: 128 us of a 20,000-splat 640x360 frame. The block stops
+// when no pixel is still accumulating (the reference's double-buffered
+// tile_alive vote), a warp when none of its own is. Output is RGBA8 packed in
+// u32 rows padded to 64 pixels, optionally also RGBA f32. A block never exits
+// with a copy still in flight into its shared memory.
 #include "kernels.h"
 
 namespace cgs {
 namespace {
 
-constexpr int kBatch = 256;
+constexpr int kBatch = 128;
+constexpr float kCut = 0.003921569f;  // 1/255
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
@@ -71,16 +81,57 @@ __global__ void k_drill_mbarrier(uint32_t* status_word, uint32_t limit) {
   if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, limit)) atomicOr(status_word, kStatusBarrierTimeout);
 }
 
+// The pixel blocks (8x4 pixels, BX by BY of them from pixel (x0, y0)) that a
+// splat can touch, one bit each: those that overlap the box of its extents.
+// Outside that box the quadratic exceeds the splat's cut; the margin of a
+// pixel plus the rounding of its three terms relative to their sum (they
+// cancel for long diagonal splats: kappa = a c / (a c - b^2)) covers the
+// computed value. Extents clamped to 1,024 bound nothing, and a conic that is
+// not finite and positive definite may pass anywhere: all blocks.
+template <uint32_t BX, uint32_t BY>
+__device__ __forceinline__ uint32_t block_mask(const float4 geo, const float4 cc, float x0, float y0) {
+  if (!(cc.y > kCut)) return 0u;  // the opacity cut
+  constexpr uint32_t kAll = BX * BY >= 32 ? 0xffffffffu : (1u << (BX * BY)) - 1u;
+  const uint32_t p = __float_as_uint(cc.w);
+  const float ex = (float)(p & 0xFFFFu), ey = (float)((p >> 16) & 0xFFFFu);
+  const float ac = geo.z * cc.x, det = ac - geo.w * geo.w;
+  const float rel = 2e-6f * (ac / fmaxf(det, 1e-7f * ac));
+  const bool fin = fabsf(geo.x) < 1e9f && fabsf(geo.y) < 1e9f && geo.z > 0.0f && cc.x > 0.0f &&
+                   det > 0.0f && ac < 1e30f;
+  if (!fin) return kAll;
+  const float hx = ex + 1.0f + ex * rel + 1e-6f * fabsf(geo.x);
+  const float hy = ey + 1.0f + ey * rel + 1e-6f * fabsf(geo.y);
+  // blocks i with x0 + 8 i + 7.5 >= mu - h and x0 + 8 i + 0.5 <= mu + h
+  const float rx = geo.x - x0, ry = geo.y - y0;
+  int i0 = max(0, __float2int_ru((rx - hx - 7.5f) * 0.125f));
+  int i1 = min((int)BX - 1, __float2int_rd((rx + hx - 0.5f) * 0.125f));
+  int j0 = max(0, __float2int_ru((ry - hy - 3.5f) * 0.25f));
+  int j1 = min((int)BY - 1, __float2int_rd((ry + hy - 0.5f) * 0.25f));
+  if (ex >= 1024.0f) i0 = 0, i1 = (int)BX - 1;
+  if (ey >= 1024.0f) j0 = 0, j1 = (int)BY - 1;
+  if (i0 > i1 || j0 > j1) return 0u;
+  const uint32_t row = ((2u << i1) - 1u) & ~((1u << i0) - 1u);
+  uint32_t m = 0;
+#pragma unroll
+  for (int j = 0; j < (int)BY; ++j)
+    if (j >= j0 && j <= j1) m |= row << (j * BX);
+  return m;
+}
+
 template <int LW, int LH>
 __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArgs a) {
   constexpr uint32_t TW = 1u << LW, TH = 1u << LH, kCompThreads = TW * TH;
-  __shared__ __align__(128) SplatRec s_rec[2][kBatch];
+  constexpr uint32_t BX = TW / 8, BY = TH / 4, NW = kCompThreads / 32;
+  static_assert(BX * BY == NW, "a warp per 8x4 pixels");
+  // [kBatch]: a record of opacity 0 that fills up a group of four
+  __shared__ __align__(128) SplatRec s_rec[2][kBatch + 1];
+  __shared__ uint32_t s_bits[kBatch / 32][NW];  // entries of a batch per warp
 
-  const uint32_t tid = threadIdx.x;
-  const uint32_t px = blockIdx.x * TW + (tid & (TW - 1u));
-  const uint32_t py = blockIdx.y * TH + (tid >> LW);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  const uint32_t tile_id = blockIdx.x, tx = tile_id % a.tiles_x, ty = tile_id / a.tiles_x;
+  const uint32_t px = tx * TW + (warp % BX) * 8u + (lane & 7u);
+  const uint32_t py = ty * TH + (warp / BX) * 4u + (lane >> 3);
   const bool inside = px < a.width && py < a.height;
-  const uint32_t tile_id = blockIdx.y * a.tiles_x + blockIdx.x;
   const uint32_t rs = min(a.ranges[2 * (size_t)tile_id], a.num_entries);
   const uint32_t re = min(a.ranges[2 * (size_t)tile_id + 1], a.num_entries);
   const bool empty = rs >= re;
@@ -105,31 +156,14 @@ __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArg
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
 
-  // Per-thread pixel state. Pixels still accumulating are re-packed into the
-  // lowest threads at every batch boundary (when that frees whole warps), so
-  // warps whose pixels have all saturated stop issuing instructions.
-  __shared__ uint32_t s_pix[kCompThreads];
-  __shared__ float4 s_acc[kCompThreads];
-  __shared__ uint32_t s_warp_alive[kCompThreads / 32];
-  int pix = inside ? (int)tid : -1;
-  bool alive = inside;
-  float cr = 0.0f, cg = 0.0f, cb = 0.0f, t = 1.0f;
-  float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
-
-  auto finalize = [&](int p, float r_, float g_, float b_, float t_) {
-    const uint32_t x = blockIdx.x * TW + ((uint32_t)p & (TW - 1u));
-    const uint32_t y = blockIdx.y * TH + ((uint32_t)p >> LW);
-    const float fr = clampf(r_ + t_ * a.bg[0], 0.0f, 1.0f);
-    const float fg = clampf(g_ + t_ * a.bg[1], 0.0f, 1.0f);
-    const float fb = clampf(b_ + t_ * a.bg[2], 0.0f, 1.0f);
-    const float fa = empty ? a.bg[3] : clampf(1.0f - t_, 0.0f, 1.0f);
-    const uint32_t r8 = (uint32_t)clampf(rintf(fr * 255.0f), 0.0f, 255.0f);
-    const uint32_t g8 = (uint32_t)clampf(rintf(fg * 255.0f), 0.0f, 255.0f);
-    const uint32_t b8 = (uint32_t)clampf(rintf(fb * 255.0f), 0.0f, 255.0f);
-    const uint32_t a8 = (uint32_t)clampf(rintf(fa * 255.0f), 0.0f, 255.0f);
-    a.out_rgba8[(size_t)y * a.pitch_px + x] = r8 | (g8 << 8) | (b8 << 16) | (a8 << 24);
-    if (a.out_f32) a.out_f32[(size_t)y * a.width + x] = make_float4(fr, fg, fb, fa);
-  };
+  // T = 0: saturated, or no pixel of the frame
+  float cr = 0.0f, cg = 0.0f, cb = 0.0f, t = inside ? 1.0f : 0.0f;
+  if (tid < 2) {
+    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    s_rec[tid][kBatch].geo = s_rec[tid][kBatch].cc = s_rec[tid][kBatch].rgb = z;
+  }
+  const float pcx = (float)px + 0.5f, pcy = (float)py + 0.5f;
+  const float bx0 = (float)(tx * TW), by0 = (float)(ty * TH);
 
   uint32_t issued = 0;
   if (nb > 0) {
@@ -150,85 +184,86 @@ __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArg
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const uint32_t cnt = min((uint32_t)kBatch, n - b * kBatch);
-    if (alive) {
-      const SplatRec* recs = s_rec[stage];
-      for (uint32_t k = 0; k < cnt; ++k) {
-        const float4 cc4 = recs[k].cc;
-        const float op = cc4.y;
-        if (op > 0.003921569f) {
-          const float4 geo = recs[k].geo;
+    const uint32_t chunks = (cnt + 31u) / 32u;
+    const SplatRec* recs = s_rec[stage];
+    for (uint32_t c = warp; c < chunks; c += NW) {
+      const uint32_t k = 32u * c + lane;
+      const uint32_t m = k < cnt ? block_mask<BX, BY>(recs[k].geo, recs[k].cc, bx0, by0) : 0u;
+      uint32_t mine = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < NW; ++w) {
+        const uint32_t v = __ballot_sync(0xffffffffu, (m >> w) & 1u);
+        if (lane == w) mine = v;
+      }
+      if (lane < NW) s_bits[c][lane] = mine;
+    }
+    __syncthreads();
+    // a lane leaves once its pixel has saturated, a warp with its last
+    for (uint32_t c = 0; c < chunks && t > 0.0f; ++c) {
+      uint32_t bits = s_bits[c][warp];
+      while (bits && t > 0.0f) {
+        uint32_t k[4];
+        float s[4], q[4], raw[4];
+        bool near = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          k[i] = bits ? 32u * c + (uint32_t)__ffs(bits) - 1u : (uint32_t)kBatch;
+          bits &= bits - 1u;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float4 cc4 = recs[k[i]].cc, geo = recs[k[i]].geo;
+          // The quadratic rounded term by term in the reference's order, so
+          // that the q >= -4 cut (q = -quad / 2, clamped to <= 0: a quad above
+          // 8 fails) agrees exactly with the host restatement.
           const float dx = pcx - geo.x, dy = pcy - geo.y;
-          // q rounded term by term in the reference's order: the q >= -4 cut
-          // then agrees exactly with the host restatement.
           const float qa = __fmul_rn(__fmul_rn(geo.z, dx), dx);
           const float qb = __fmul_rn(__fmul_rn(__fmul_rn(2.0f, geo.w), dx), dy);
           const float qc = __fmul_rn(__fmul_rn(cc4.x, dy), dy);
-          float q = __fmul_rn(-0.5f, __fadd_rn(__fadd_rn(qa, qb), qc));
-          q = fminf(q, 0.0f);
-          if (q >= -4.0f) {
-            float raw = op * __expf(q);
-            // Near the 1/255 visibility cut, re-evaluate with the deterministic
-            // exp so the keep/skip decision matches the host restatement.
-            if (fabsf(raw - 0.003921569f) < 4e-7f) raw = __fmul_rn(op, cgs_expf(q));
-            const float alpha = fminf(0.99f, raw);
-            if (alpha >= 0.003921569f) {
-              const float4 rgb = recs[k].rgb;
-              const float w = alpha * t;
-              cr += w * rgb.x;
-              cg += w * rgb.y;
-              cb += w * rgb.z;
-              t *= 1.0f - alpha;
-              if (t < 0.001f) {
-                alive = false;
-                t = 0.0f;
-                break;
-              }
-            }
-          }
+          s[i] = __fadd_rn(__fadd_rn(qa, qb), qc);
+          q[i] = fminf(__fmul_rn(-0.5f, s[i]), 0.0f);
+          raw[i] = cc4.y * __expf(q[i]);
+          near = near || fabsf(raw[i] - kCut) < 4e-7f;
+        }
+        // Near the 1/255 visibility cut, re-evaluate with the deterministic
+        // exp so the keep/skip decision matches the host restatement.
+        if (near) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (fabsf(raw[i] - kCut) < 4e-7f) raw[i] = __fmul_rn(recs[k[i]].cc.y, cgs_expf(q[i]));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          float alpha = fminf(0.99f, raw[i]);
+          alpha = alpha >= kCut && !(s[i] > 8.0f) ? alpha : 0.0f;
+          const float4 rgb = recs[k[i]].rgb;
+          const float w = alpha * t;
+          cr += w * rgb.x;
+          cg += w * rgb.y;
+          cb += w * rgb.z;
+          t *= 1.0f - alpha;
+          if (t < 0.001f) t = 0.0f;
         }
       }
     }
-    // Batch boundary: write finished pixels, stop when none is left, and
-    // re-pack the survivors when they are spread over more warps than needed.
-    if (pix >= 0 && !alive) {
-      finalize(pix, cr, cg, cb, t);
-      pix = -1;
-    }
-    const uint32_t lane = tid & 31u, warp = tid >> 5;
-    const uint32_t wmask = __ballot_sync(0xffffffffu, alive);
-    const int n_alive = __syncthreads_count(alive);
-    if (n_alive == 0) break;
-    const int warps_busy = __syncthreads_count(lane == 0 && wmask != 0u);
-    if (b + 1 < nb && warps_busy > (n_alive + 31) / 32) {
-      if (lane == 0) s_warp_alive[warp] = __popc(wmask);
-      __syncthreads();
-      uint32_t base = 0;
-      for (uint32_t w = 0; w < warp; ++w) base += s_warp_alive[w];
-      if (alive) {
-        const uint32_t slot = base + __popc(wmask & lanemask_lt());
-        s_pix[slot] = (uint32_t)pix;
-        s_acc[slot] = make_float4(cr, cg, cb, t);
-      }
-      __syncthreads();
-      alive = (int)tid < n_alive;
-      if (alive) {
-        pix = (int)s_pix[tid];
-        const float4 acc = s_acc[tid];
-        cr = acc.x;
-        cg = acc.y;
-        cb = acc.z;
-        t = acc.w;
-        pcx = (float)(blockIdx.x * TW + ((uint32_t)pix & (TW - 1u))) + 0.5f;
-        pcy = (float)(blockIdx.y * TH + ((uint32_t)pix >> LW)) + 0.5f;
-      } else {
-        pix = -1;
-      }
-    }
+    // Batch boundary: stop when no pixel is left (also orders this batch's
+    // reads before the copies that refill its buffer).
+    if (!__syncthreads_or(t > 0.0f)) break;
   }
   // Never leave with a copy still writing into this block's shared memory.
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   if (tid == 0 && a.fc && issued > 0) atomicAdd(&a.fc->fetched, min(n, issued * (uint32_t)kBatch));
-  if (pix >= 0) finalize(pix, cr, cg, cb, t);
+  if (!inside) return;
+  const float fr = clampf(cr + t * a.bg[0], 0.0f, 1.0f);
+  const float fg = clampf(cg + t * a.bg[1], 0.0f, 1.0f);
+  const float fb = clampf(cb + t * a.bg[2], 0.0f, 1.0f);
+  const float fa = empty ? a.bg[3] : clampf(1.0f - t, 0.0f, 1.0f);
+  const uint32_t r8 = (uint32_t)clampf(rintf(fr * 255.0f), 0.0f, 255.0f);
+  const uint32_t g8 = (uint32_t)clampf(rintf(fg * 255.0f), 0.0f, 255.0f);
+  const uint32_t b8 = (uint32_t)clampf(rintf(fb * 255.0f), 0.0f, 255.0f);
+  const uint32_t a8 = (uint32_t)clampf(rintf(fa * 255.0f), 0.0f, 255.0f);
+  a.out_rgba8[(size_t)py * a.pitch_px + px] = r8 | (g8 << 8) | (b8 << 16) | (a8 << 24);
+  if (a.out_f32) a.out_f32[(size_t)py * a.width + px] = make_float4(fr, fg, fb, fa);
 }
 
 }  // namespace
@@ -240,13 +275,13 @@ cudaError_t launch_drill_mbarrier(uint32_t* status_word, uint32_t limit, cudaStr
 
 cudaError_t launch_composite(const CompositeArgs& a, cudaStream_t s) {
   if (a.tiles_x == 0 || a.tiles_y == 0) return cudaSuccess;
-  dim3 grid(a.tiles_x, a.tiles_y);
+  const uint32_t tiles = a.tiles_x * a.tiles_y;
   if (a.tile_w_log2 == 3 && a.tile_h_log2 == 3)
-    k_composite<3, 3><<<grid, 64, 0, s>>>(a);
+    k_composite<3, 3><<<tiles, 64, 0, s>>>(a);
   else if (a.tile_w_log2 == 5 && a.tile_h_log2 == 4)
-    k_composite<5, 4><<<grid, 512, 0, s>>>(a);
+    k_composite<5, 4><<<tiles, 512, 0, s>>>(a);
   else if (a.tile_w_log2 == 4 && a.tile_h_log2 == 4)
-    k_composite<4, 4><<<grid, 256, 0, s>>>(a);
+    k_composite<4, 4><<<tiles, 256, 0, s>>>(a);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();

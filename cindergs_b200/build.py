@@ -41,7 +41,7 @@ UNITS = [
     ("pipeline.cu", []),
     ("noalloc.cu", []),
 ]
-HEADERS = ["common.cuh", "detmath.h", "kernels.h", "field.h", "tile_test.cuh"]
+HEADERS = ["common.cuh", "detmath.h", "kernels.h", "field.h", "tile_test.cuh", "tile_span.h"]
 
 
 def _nvcc() -> str:

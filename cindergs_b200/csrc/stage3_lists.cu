@@ -11,22 +11,21 @@
 //                 average at 1080p, where it touches 24 tiles); one
 //                 (block, splat) pair per touched block is written in slot order;
 //   (pair sort):  stable radix sort of the pairs by block;
-//   k_list_count: a warp takes 32 pairs of one block, one per lane, and runs
-//                 the exact ellipse-vs-tile test against the block's 32 tiles
-//                 in turn: the ballot of tile t's tests is tile t's list of
-//                 these 32 splats, already in depth order;
+//   k_list_count: a warp takes 32 pairs of one block, one per lane, finds the
+//                 tiles of the block each hits (an interval of columns per
+//                 row) and transposes the 32 words: tile t's word is its list
+//                 of these 32 splats, already in depth order;
 //   k_list_place: each chunk's first entry per tile inside its block, the
 //                 tiles' first entries and their [start, end) ranges;
-//   k_list_write: every ballot's splats are stored at their places.
+//   k_list_write: every word's splats are stored at their places.
 //
-// An entry costs one ballot bit and one 4-byte store instead of a 4-byte key
+// An entry costs one bit and one 4-byte store instead of a 4-byte key
 // and a 4-byte index written by the binning and moved by two or three radix
-// passes; the tests need no owner search, no tables and no look-back. The
-// block shape balances the tests wasted on tiles outside a splat's box (32
-// per pair) against the pairs: 8x8-tile blocks tested 1.7 times as many.
+// passes, and nothing is evaluated per tile.
 #include <algorithm>
 
 #include "kernels.h"
+#include "tile_span.h"
 #include "tile_test.cuh"
 
 namespace cgs {
@@ -188,72 +187,56 @@ __device__ __forceinline__ uint32_t block_of(const uint32_t* first, uint32_t nb,
   return lo;
 }
 
-// Two binary32 values in one register pair: sm_100's packed products and sums
-// round each half as the scalar instructions do. A packed product that feeds
-// a packed sum is contracted into one fused operation whatever its rounding
-// qualifier and -fmad say, which changes the test's result now and then (one
-// entry in 3 million of a 2400x1800 frame with 8x8 tiles). Such products are
-// written as a b + z instead, z = -0 from a kernel argument the compiler
-// cannot see through: exactly the rounded product, and nothing to contract.
-using f2 = unsigned long long;
-__device__ __forceinline__ f2 pack2(float lo, float hi) {
-  f2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-  f2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-  f2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-  f2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
+// ellipse_intersects_tile_gpu (binning.rs:37-96) for tile (tx, ty), every
+// operation rounded separately in the reference's operand order (a call: only
+// the tiles that tile_span.h leaves undecided come here).
+__device__ __noinline__ bool tile_exact(uint32_t tx, uint32_t ty, uint32_t lw, uint32_t lh, uint32_t wm1,
+                                        uint32_t hm1, float mu_x, float mu_y, float a, float b, float c,
+                                        float lim) {
+  const uint32_t xs = tx << lw, ys = ty << lh;
+  const float dx0 = __fsub_rn(pixel_center(xs), mu_x);
+  const float dx1 = __fsub_rn(pixel_center(min(xs + ((1u << lw) - 1u), wm1)), mu_x);
+  const float dy0 = __fsub_rn(pixel_center(ys), mu_y);
+  const float dy1 = __fsub_rn(pixel_center(min(ys + ((1u << lh) - 1u), hm1)), mu_y);
+  const float b2 = __fmul_rn(2.0f, b);
+  const float xn = clampf(0.0f, dx0, dx1), yn = clampf(0.0f, dy0, dy1);
+  const float y1 = clampf(__fdiv_rn(__fmul_rn(-b, xn), fmaxf(c, 1e-12f)), dy0, dy1);
+  const float q1 = __fadd_rn(__fadd_rn(__fmul_rn(__fmul_rn(a, xn), xn), __fmul_rn(__fmul_rn(b2, xn), y1)),
+                             __fmul_rn(__fmul_rn(c, y1), y1));
+  const float x2 = clampf(__fdiv_rn(__fmul_rn(-b, yn), fmaxf(a, 1e-12f)), dx0, dx1);
+  const float q2 = __fadd_rn(__fadd_rn(__fmul_rn(__fmul_rn(a, x2), x2), __fmul_rn(__fmul_rn(b2, x2), yn)),
+                             __fmul_rn(__fmul_rn(c, yn), yn));
+  return fminf(q1, q2) <= lim;
 }
 
-// n / d in both halves, correctly rounded to binary32, from y = RN(1 / d):
-// Markstein's division (IBM J. Res. Dev. 34(1), 1990). One step makes q
-// faithful; from a faithful q and a correctly rounded reciprocal the second
-// gives the correctly rounded quotient, as long as nothing under- or
-// overflows (3 x 10^9 operand pairs equal n / d). The sign of a zero is lost.
-__device__ __forceinline__ f2 div2(f2 n, f2 neg_d, f2 y) {
-  const f2 q = mul2(n, y);
-  const f2 q1 = fma2(fma2(neg_d, q, n), y, q);
-  return fma2(fma2(neg_d, q1, n), y, q1);
-}
-__device__ __noinline__ f2 div2_ieee(f2 n, f2 neg_d) {
-  float a, b, c, d;
-  unpack2(n, a, b);
-  unpack2(neg_d, c, d);
-  return pack2(__fdiv_rn(a, -c), __fdiv_rn(b, -d));
+// Transpose of a 32x32 bit matrix, a row per lane: lane t gets bit t of every
+// lane's word, lane l's at bit l.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
+  uint32_t m = 0x0000FFFFu;
+#pragma unroll
+  for (int j = 16; j >= 1; j >>= 1) {
+    const uint32_t y = __shfl_xor_sync(0xffffffffu, x, j);
+    x = (lane & j) ? ((x & ~m) | ((y >> j) & m)) : ((x & m) | ((y & m) << j));
+    m ^= m << (j >> 1);
+  }
+  return x;
 }
 
-// The tests of 32 pairs of a block against its 32 tiles, one pair per lane
-// (ellipse_intersects_tile_gpu, binning.rs:37-96, term for term). Per lane the
-// four rows' terms stay in registers and the eight columns are walked two at a
-// time; a tile takes two clamps, a compare pair and half of 11 packed products
-// and sums, then one ballot. A tile outside the lane's own tile box fails: its
-// row's limit is NaN, its column's predicate false. Bound by instruction issue
-// (clamps and compares run at half the products' rate).
-__global__ void __launch_bounds__(kListThreads, 3) k_list_count(const ListArgs a, float neg_zero) {
-  __shared__ __align__(16) uint32_t s_mask[kListWarps][32];
+// The tiles that 32 pairs of a block hit, one pair per lane: for each of the
+// block's four rows the columns the splat's ellipse reaches (tile_span.h), and
+// the test itself for the few tiles that lie within the rounding margin of
+// an end; the 32 lanes' words are then transposed into the 32 tiles' lists.
+// One interval per row instead of eight tests: 880 -> 590 instructions per 32
+// pairs, 168 -> 113 us at 4.4M pairs (1.1M splats, 1080p). Bound by
+// instruction issue.
+__global__ void __launch_bounds__(kListThreads) k_list_count(const ListArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunks = a.plan->chunks, groups = a.plan->groups;
   const uint32_t active = min(a.n_rest + (a.split_count ? *a.split_count : 0u), a.max_n);
-  const float x_last = pixel_center(a.width - 1u), y_last = pixel_center(a.height - 1u);
+  const uint32_t wm1 = a.width - 1u, hm1 = a.height - 1u;
+  const float x_last = pixel_center(wm1), y_last = pixel_center(hm1);
   const uint32_t lw = a.tile_w_log2, lh = a.tile_h_log2;
   const float tw = (float)(1u << lw), th = (float)(1u << lh);
-  uint32_t* sm = s_mask[warp];
-  const f2 nz = pack2(neg_zero, neg_zero);
   for (uint32_t c = blockIdx.x * kListWarps + warp; c < chunks; c += gridDim.x * kListWarps) {
     const uint32_t b = block_of(a.chunk_first, a.num_blocks, c);
     const uint32_t tx0 = (b % a.blocks_x) << kListBlockW, ty0 = (b / a.blocks_x) << kListBlockH;
@@ -268,83 +251,33 @@ __global__ void __launch_bounds__(kListThreads, 3) k_list_count(const ListArgs a
       const float lim = bx.valid ? a.recs[sid].rgb.w : 0.0f;
       const uint32_t nxt = i0 + 32u * (j + 1) + lane;
       sid = j + 1 < groups && nxt < end ? a.sorted_pairs[nxt] : kInvalid;
-      const float nan = __int_as_float(0x7FC00000);
-      const float ca_ = fmaxf(bx.ca, 1e-12f), cc_ = fmaxf(bx.cc, 1e-12f);
-      const float cb2 = __fmul_rn(2.0f, bx.cb);
-      const float ya = __frcp_rn(ca_), yc = __frcp_rn(cc_);
-      // a nonzero distance to a pixel centre is at least 2^-25 and below 2^24,
-      // so with these bounds no quotient or residue leaves the normal range
-      const bool ok = (bx.cb == 0.0f || fabsf(bx.cb) >= 0x1p-30f) && fabsf(bx.cb) < 0x1p40f &&
-                      ca_ <= 0x1p20f && cc_ <= 0x1p20f;
-      const bool fast = __all_sync(0xffffffffu, ok || !bx.valid);
-      const f2 ca2 = pack2(bx.ca, bx.ca), cc2 = pack2(bx.cc, bx.cc), cb22 = pack2(cb2, cb2);
-      const f2 nb2 = pack2(-bx.cb, -bx.cb);
-      float y0[4], y1[4], rz[4], rl[4];
-      f2 yn[4], rw[4];
-      {
-        const f2 nmu = pack2(-bx.mu_y, -bx.mu_y), nd = pack2(-ca_, -ca_), y2 = pack2(ya, ya);
+      const float dx00 = px0 - bx.mu_x;
+      const SplatSpan sp = splat_span(bx.ca, bx.cb, bx.cc, lim, dx00, (px0 + (tw - 1.0f)) - bx.mu_x,
+                                      x_last - bx.mu_x, tw);
+      // the splat's tile box in this block
+      const int c0 = max((int)bx.x0 - (int)tx0, 0), c1 = min((int)bx.x1 - (int)tx0, 7);
+      const uint32_t cols = bx.valid && c1 >= c0 ? ((2u << c1) - 1u) & ~((1u << c0) - 1u) : 0u;
+      uint32_t hits = 0, open = 0;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float f0 = py0 + (float)(2 * h) * th, f1 = f0 + th;
-          unpack2(add2(pack2(f0, f1), nmu), y0[2 * h], y0[2 * h + 1]);
-          unpack2(add2(pack2(fminf(f0 + (th - 1.0f), y_last), fminf(f1 + (th - 1.0f), y_last)), nmu),
-                  y1[2 * h], y1[2 * h + 1]);
-          const float na = clampf(0.0f, y0[2 * h], y1[2 * h]);
-          const float nb = clampf(0.0f, y0[2 * h + 1], y1[2 * h + 1]);
-          const f2 n = pack2(na, nb), num = mul2(nb2, n);
-          unpack2(fast ? div2(num, nd, y2) : div2_ieee(num, nd), rz[2 * h], rz[2 * h + 1]);
-          float wa, wb;
-          unpack2(mul2(mul2(cc2, n), n), wa, wb);
-          yn[2 * h] = pack2(na, na);
-          yn[2 * h + 1] = pack2(nb, nb);
-          rw[2 * h] = pack2(wa, wa);
-          rw[2 * h + 1] = pack2(wb, wb);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          rl[k] = bx.valid && ty0 + k >= bx.y0 && ty0 + k <= bx.y1 ? lim : nan;
+      for (uint32_t r = 0; r < 4; ++r) {
+        const float f = py0 + (float)r * th;
+        uint32_t in, out;
+        row_span(sp, f - bx.mu_y, fminf(f + (th - 1.0f), y_last) - bx.mu_y, in, out);
+        const uint32_t row = ty0 + r >= bx.y0 && ty0 + r <= bx.y1 ? cols : 0u;
+        hits |= (sp.ok ? in & row : 0u) << (8u * r);
+        open |= (sp.ok ? out & ~in & row : row) << (8u * r);
       }
-      const f2 nmu = pack2(-bx.mu_x, -bx.mu_x), nd = pack2(-cc_, -cc_), y2 = pack2(yc, yc);
-#pragma unroll 1
-      for (uint32_t k = 0; k < 8; k += 2) {
-        const uint32_t tx = tx0 + k;
-        const bool in0 = tx >= bx.x0 && tx <= bx.x1, in1 = tx + 1 >= bx.x0 && tx + 1 <= bx.x1;
-        const float f0 = px0 + (float)k * tw, f1 = f0 + tw;
-        float x0a, x0b, x1a, x1b;
-        unpack2(add2(pack2(f0, f1), nmu), x0a, x0b);
-        unpack2(add2(pack2(fminf(f0 + (tw - 1.0f), x_last), fminf(f1 + (tw - 1.0f), x_last)), nmu), x1a,
-                x1b);
-        const f2 xn = pack2(clampf(0.0f, x0a, x1a), clampf(0.0f, x0b, x1b));
-        const f2 num = mul2(nb2, xn);
-        float cza, czb;
-        unpack2(fast ? div2(num, nd, y2) : div2_ieee(num, nd), cza, czb);
-        const f2 cw = fma2(mul2(ca2, xn), xn, nz);
-        const f2 cp = mul2(cb22, xn);
-        uint32_t m0[4], m1[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const f2 y = pack2(clampf(cza, y0[r], y1[r]), clampf(czb, y0[r], y1[r]));
-          const f2 q1 = add2(add2(cw, fma2(cp, y, nz)), fma2(mul2(cc2, y), y, nz));
-          const f2 x = pack2(clampf(rz[r], x0a, x1a), clampf(rz[r], x0b, x1b));
-          const f2 q2 = add2(add2(fma2(mul2(ca2, x), x, nz), fma2(mul2(cb22, x), yn[r], nz)), rw[r]);
-          float q1a, q1b, q2a, q2b;
-          unpack2(q1, q1a, q1b);
-          unpack2(q2, q2a, q2b);
-          // fminf(q1, q2) <= limit: either is (a NaN never is)
-          m0[r] = __ballot_sync(0xffffffffu, in0 && (q1a <= rl[r] || q2a <= rl[r]));
-          m1[r] = __ballot_sync(0xffffffffu, in1 && (q1b <= rl[r] || q2b <= rl[r]));
-        }
-        if (lane == 0) {
-          *reinterpret_cast<uint4*>(sm + 4 * k) = make_uint4(m0[0], m0[1], m0[2], m0[3]);
-          *reinterpret_cast<uint4*>(sm + 4 * k + 4) = make_uint4(m1[0], m1[1], m1[2], m1[3]);
-        }
+      while (open) {
+        const uint32_t t = (uint32_t)__ffs(open) - 1u;
+        open &= open - 1u;
+        if (tile_exact(tx0 + (t & 7u), ty0 + (t >> 3), lw, lh, wm1, hm1, bx.mu_x, bx.mu_y, bx.ca, bx.cb,
+                       bx.cc, lim))
+          hits |= 1u << t;
       }
       __syncwarp();
-      // lane t holds tile t (row-major in the block)
-      const uint32_t mt = sm[(lane & 7) * 4 + (lane >> 3)];
+      const uint32_t mt = transpose_bits(hits, lane);
       a.masks[((size_t)c * groups + j) * 32 + lane] = mt;
       cnt += __popc(mt);
-      __syncwarp();
     }
     a.chunk_base[(size_t)c * 32 + lane] = cnt;
   }
@@ -540,7 +473,7 @@ cudaError_t launch_list_pairs(const ListArgs& a, cudaStream_t s) {
 cudaError_t launch_list_count(const ListArgs& a, cudaStream_t s) {
   static const uint32_t grid = resident_blocks(k_list_count, kListThreads);
   const uint32_t most = (list_chunk_cap(a.pair_cap, a.num_blocks) + kListWarps - 1) / kListWarps;
-  k_list_count<<<std::min(most, grid), kListThreads, 0, s>>>(a, -0.0f);
+  k_list_count<<<std::min(most, grid), kListThreads, 0, s>>>(a);
   return cudaGetLastError();
 }
 

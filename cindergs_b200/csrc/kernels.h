@@ -430,7 +430,8 @@ struct SortArgs {
   uint32_t* keys[2];     // ping-pong key buffers
   uint32_t* vals[2];     // ping-pong payload word 0
   uint32_t* vals2[2];    // ping-pong payload word 1 (null for one-word payloads)
-  const uint32_t* n_ptr; // device element count (may exceed capacity -> capacity flag)
+  const uint32_t* n_ptr; // device element count (may exceed capacity -> capacity flag), or
+                         // null: capacity elements
   uint32_t capacity;     // elements the buffers hold; grid is sized for it
   uint32_t first_bit;    // lowest key bit to sort on
   uint32_t num_bits;     // bits to sort on (from first_bit)

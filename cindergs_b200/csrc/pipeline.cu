@@ -3364,11 +3364,10 @@ static int sort_common(cgs_ctx* ctx, uint32_t* d_keys, uint32_t* d_vals, uint32_
   if (d_vals2) CGS_TRY(ctx->ensure(ctx->prim[3], (size_t)n * 4, "sort alt values"));
   char* b = ctx->prim[0].as<char>();
   CGS_CUDA(cudaMemsetAsync(b, 0, bytes, ctx->stream), "clear sort scratch");
-  uint32_t* words = (uint32_t*)b;  // [0] n, [1] status, [2..] tile counters
+  uint32_t* words = (uint32_t*)b;  // [1] status, [2..] tile counters
   const uint32_t n32 = (uint32_t)n;
-  CGS_CUDA(cudaMemcpyAsync(words, &n32, 4, cudaMemcpyHostToDevice, ctx->stream), "sort n");
   uint32_t* hist = (uint32_t*)(b + 256);
-  CGS_CUDA(launch_histogram(d_keys, words, n32, 0, key_bits, rb, hist, ctx->stream), "histogram");
+  CGS_CUDA(launch_histogram(d_keys, nullptr, n32, 0, key_bits, rb, hist, ctx->stream), "histogram");
   SortArgs sa{};
   sa.keys[0] = d_keys;
   sa.keys[1] = ctx->prim[1].as<uint32_t>();
@@ -3378,10 +3377,12 @@ static int sort_common(cgs_ctx* ctx, uint32_t* d_keys, uint32_t* d_vals, uint32_
     sa.vals2[0] = d_vals2;
     sa.vals2[1] = ctx->prim[3].as<uint32_t>();
   }
-  sa.n_ptr = words;
   sa.capacity = n32;
   sa.first_bit = 0;
   sa.num_bits = key_bits;
+  // arbitrary keys: a warp's 32 digits are mostly different (48 us a pass of 3M
+  // pairs with one ballot per digit bit)
+  sa.smem_mask = ~0u;
   sa.radix_bits = rb;
   sa.hist = hist;
   sa.status = b + hdr;

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(kSortThreads, PAY2 ? 3 : 4) k_onesweep(const P
   uint32_t* s_wor = s_misc + 48;                 // [warps][3][R] peer masks (kRankSmem)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  uint32_t n = *a.n_ptr;
+  uint32_t n = a.n_ptr ? *a.n_ptr : a.capacity;
   if (n > a.capacity) n = a.capacity;
   const uint32_t num_tiles = (n + kSortTile - 1) / kSortTile;
   if (tid == 0) s_misc[0] = atomicAdd(a.tile_ctr, 1u);
@@ -367,7 +367,7 @@ __global__ void k_histogram(const uint32_t* __restrict__ keys, const uint32_t* _
   const uint32_t passes = (num_bits + radix_bits - 1) / radix_bits;
   for (uint32_t k = threadIdx.x; k < passes * R; k += blockDim.x) s_hist[k] = 0u;
   __syncthreads();
-  uint32_t n = *n_ptr;
+  uint32_t n = n_ptr ? *n_ptr : capacity;
   if (n > capacity) n = capacity;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint32_t key = keys[i];

@@ -360,49 +360,73 @@ __global__ void __launch_bounds__(256) k_field_update(FieldUpdate a) {
 
 // ---- frame: per-frame projection and fused inference ---------------------------
 
-// Per-frame projection of the output layer (one block of 1024 threads). For
+// Per-frame projection of the output layer. For
 // vertices u (rest or current), P_u[k] = sum_j W5[j][k] u_j - c_k ubar with
 // c_k = sum_j W5[j][k], and p0_u = sum_j b5_j u_j + (1 - sum_j b5_j) ubar, so
 // that sum_j w0_j u_j = P_u^T h + p0_u. Raw mode (verts == null): P_rest,
 // p0_rest and A3 = 0, i.e. the network's own rest position sum_j w0_j v_j.
 // Otherwise A = v'^T Vb^T M, Pc = P_cur - P_rest A3^T, pc = p0_cur - A3 p0_rest.
 // proj = [Pc (128 x 3) | pc (3) | A3 (3 x 3, row-major)]. Both vertex sets
-// are staged in shared memory; thread (g, k) sums vertices j = g mod 8 for
-// hidden unit k and the eight partial sums are added in g order.
-constexpr int kProjThreads = 1024, kProjGroups = kProjThreads / kHid;
+// are staged in shared memory; the vertices j = g mod 8 are summed per hidden
+// unit and the eight partial sums are added in g order. Each of 16 blocks of
+// 1024 threads takes eight hidden units, their columns of W5 staged with one
+// 16-byte load per vertex, and repeats the 22 sums over the vertices, a
+// warp's sums per value added by one lane (one block that did all of it, with
+// every thread adding every warp's sums, took 32 us at 642 vertices; latency
+// bounds it).
+constexpr int kProjThreads = 1024, kProjGroups = 8, kProjUnits = 8;
 __global__ void __launch_bounds__(kProjThreads) k_field_project(FieldNet net, uint32_t V,
                                                                 const float4* __restrict__ rest,
                                                                 const float4* __restrict__ verts,
                                                                 const float* __restrict__ M,
                                                                 float* __restrict__ proj) {
-  extern __shared__ float4 pv[];  // [V] rest, [V] current
+  extern __shared__ float4 pv[];  // [V] rest, [V] current, [V] this block's columns of W5
   __shared__ float red[22 * 32];
-  __shared__ float part[kProjGroups][7][kHid];
-  __shared__ float sh[20];
+  __shared__ float part[kProjGroups][7][kProjUnits];
+  __shared__ float sh[20], t[22];
+  const uint32_t k0 = blockIdx.x * kProjUnits;
   const bool raw = verts == nullptr;
   for (uint32_t j = threadIdx.x; j < V; j += blockDim.x) {
     pv[j] = rest[j];
     pv[V + j] = raw ? make_float4(0.f, 0.f, 0.f, 0.f) : verts[j];
+    pv[2 * V + j] = *reinterpret_cast<const float4*>(net.W5b + (size_t)j * kHid + k0);
   }
   __syncthreads();
   // sums: rest (3), rest . b5 (3), sum b5 (1), current (3), current . b5 (3),
   // sum_j v'_j v_j^T (9)
-  float t[22];
+  float v_[22];
 #pragma unroll
-  for (int k = 0; k < 22; ++k) t[k] = 0.0f;
+  for (int k = 0; k < 22; ++k) v_[k] = 0.0f;
   for (uint32_t j = threadIdx.x; j < V; j += blockDim.x) {
     const float4 v = pv[j], c = pv[V + j];
     const float b = net.b5[j];
-    t[0] += v.x; t[1] += v.y; t[2] += v.z;
-    t[3] += b * v.x; t[4] += b * v.y; t[5] += b * v.z;
-    t[6] += b;
-    t[7] += c.x; t[8] += c.y; t[9] += c.z;
-    t[10] += b * c.x; t[11] += b * c.y; t[12] += b * c.z;
-    t[13] += c.x * v.x; t[14] += c.x * v.y; t[15] += c.x * v.z;
-    t[16] += c.y * v.x; t[17] += c.y * v.y; t[18] += c.y * v.z;
-    t[19] += c.z * v.x; t[20] += c.z * v.y; t[21] += c.z * v.z;
+    v_[0] += v.x; v_[1] += v.y; v_[2] += v.z;
+    v_[3] += b * v.x; v_[4] += b * v.y; v_[5] += b * v.z;
+    v_[6] += b;
+    v_[7] += c.x; v_[8] += c.y; v_[9] += c.z;
+    v_[10] += b * c.x; v_[11] += b * c.y; v_[12] += b * c.z;
+    v_[13] += c.x * v.x; v_[14] += c.x * v.y; v_[15] += c.x * v.z;
+    v_[16] += c.y * v.x; v_[17] += c.y * v.y; v_[18] += c.y * v.z;
+    v_[19] += c.z * v.x; v_[20] += c.z * v.y; v_[21] += c.z * v.z;
   }
-  block_sums<22>(t, red);
+  {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 22; ++k)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v_[k] += __shfl_xor_sync(0xffffffffu, v_[k], o);
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < 22; ++k) red[k * 32 + warp] = v_[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 22) {
+    float x = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 32; ++w) x += red[threadIdx.x * 32 + w];
+    t[threadIdx.x] = x;
+  }
+  __syncthreads();
   if (threadIdx.x == 0) {
     const float inv_v = 1.0f / (float)V;
     const float rb[3] = {t[0] * inv_v, t[1] * inv_v, t[2] * inv_v};
@@ -412,9 +436,10 @@ __global__ void __launch_bounds__(kProjThreads) k_field_project(FieldNet net, ui
       sh[q] = rb[q];
       sh[3 + q] = p0r[q];
     }
+    const bool first = blockIdx.x == 0;  // writes the terms that no hidden unit has
     if (raw) {
-      for (int q = 0; q < 3; ++q) proj[3 * kHid + q] = p0r[q];
-      for (int k = 0; k < 9; ++k) proj[3 * kHid + 3 + k] = 0.0f;
+      for (int q = 0; first && q < 3; ++q) proj[3 * kHid + q] = p0r[q];
+      for (int k = 0; first && k < 9; ++k) proj[3 * kHid + 3 + k] = 0.0f;
     } else {
       const float cb[3] = {t[7] * inv_v, t[8] * inv_v, t[9] * inv_v};
       // S (3 x 4): column 0 = sum_j v'_j, columns 1..3 = sum_j v'_j v_j^T
@@ -432,29 +457,35 @@ __global__ void __launch_bounds__(kProjThreads) k_field_project(FieldNet net, ui
       for (int q = 0; q < 3; ++q) {
         sh[6 + q] = cb[q];
         const float p0c = t[10 + q] + (1.0f - t[6]) * cb[q];
-        proj[3 * kHid + q] =
-            p0c - (A3[q][0] * p0r[0] + A3[q][1] * p0r[1] + A3[q][2] * p0r[2]);
-        for (int d = 0; d < 3; ++d) proj[3 * kHid + 3 + 3 * q + d] = A3[q][d];
+        const float pc = p0c - (A3[q][0] * p0r[0] + A3[q][1] * p0r[1] + A3[q][2] * p0r[2]);
+        if (first) {
+          proj[3 * kHid + q] = pc;
+          for (int d = 0; d < 3; ++d) proj[3 * kHid + 3 + 3 * q + d] = A3[q][d];
+        }
       }
     }
   }
-  const uint32_t k = threadIdx.x % kHid, g = threadIdx.x / kHid;
+  const uint32_t kk = threadIdx.x % kProjUnits, g = threadIdx.x / kProjUnits, k = k0 + kk;
   float acc[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // rest (3), current (3), c
-  for (uint32_t j = g; j < V; j += kProjGroups) {
-    const float w = __bfloat162float(net.W5b[(size_t)j * kHid + k]);
-    const float4 v = pv[j], u = pv[V + j];
-    acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z;
-    acc[3] += w * u.x; acc[4] += w * u.y; acc[5] += w * u.z;
-    acc[6] += w;
-  }
+  if (g < kProjGroups) {
+    const __nv_bfloat16* w5 = reinterpret_cast<const __nv_bfloat16*>(pv + 2 * V);
+#pragma unroll 4
+    for (uint32_t j = g; j < V; j += kProjGroups) {
+      const float w = __bfloat162float(w5[j * kProjUnits + kk]);
+      const float4 v = pv[j], u = pv[V + j];
+      acc[0] += w * v.x; acc[1] += w * v.y; acc[2] += w * v.z;
+      acc[3] += w * u.x; acc[4] += w * u.y; acc[5] += w * u.z;
+      acc[6] += w;
+    }
 #pragma unroll
-  for (int q = 0; q < 7; ++q) part[g][q][k] = acc[q];
+    for (int q = 0; q < 7; ++q) part[g][q][kk] = acc[q];
+  }
   __syncthreads();  // also publishes sh
   if (g != 0) return;
 #pragma unroll
   for (int q = 0; q < 7; ++q) {
     float tot = 0.0f;
-    for (int gg = 0; gg < kProjGroups; ++gg) tot += part[gg][q][k];
+    for (int gg = 0; gg < kProjGroups; ++gg) tot += part[gg][q][kk];
     acc[q] = tot;
   }
   float pr[3];
@@ -721,12 +752,11 @@ cudaError_t launch_field_update(const FieldUpdate& u, cudaStream_t s) {
 cudaError_t launch_field_project(const FieldNet& net, uint32_t V, const float4* rest,
                                  const float4* verts, const float* M, float* proj,
                                  cudaStream_t s) {
-  // static shared memory (~32 KB) plus the two vertex sets
-  const size_t smem = (size_t)V * 32;
+  const size_t smem = (size_t)V * 48;
   const cudaError_t e = cudaFuncSetAttribute(
       k_field_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_field_project<<<1, kProjThreads, smem, s>>>(net, V, rest, verts, M, proj);
+  k_field_project<<<kHid / kProjUnits, kProjThreads, smem, s>>>(net, V, rest, verts, M, proj);
   return cudaGetLastError();
 }
 

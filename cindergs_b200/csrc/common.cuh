@@ -35,6 +35,8 @@ struct FrameCounters {
   uint32_t tile_ctr[16]; // dynamic tile counters for chained-scan kernels
   uint32_t pairs;        // Stage 3 (splat, screen block) pairs
   unsigned long long stage_ctr;  // binning: staged entries so far (64 bits: never wraps)
+  uint32_t written;      // screen-block lists: entries held by the id buffer
+  uint32_t pad;
 };
 // Largest tile-entry capacity of a frame (32-bit entry indices; a multiple
 // of the radix sort's 4096-entry tiles; the entry sort's look-back words are

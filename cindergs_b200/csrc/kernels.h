@@ -347,6 +347,11 @@ constexpr uint32_t kListSlots = 1024;       // slots of one pairing tile
 constexpr uint32_t kListSmallPairs = 1u << 18;  // up to here a chunk is one group of 32 pairs
 constexpr uint32_t kListGroups = 4;         // groups of 32 pairs per chunk beyond
 constexpr uint32_t kListSegChunks = 64;     // chunks of one placing segment
+// Entries of a tile that are written out: its front-most ones. A tile's pixels
+// saturate long before its list ends (after at most 420 of up to 32,000 entries
+// in a 100,000-splat 720p frame), and the compositor takes what lies beyond
+// from the blocks' hit words. A multiple of its batch.
+constexpr uint32_t kListLimit = 1024;
 // The screen blocks a splat's tile box touches: first block | width << 14 |
 // height << 23, 0 when the splat has no entries (a box spans at most 1024 + 1
 // + 1024 pixels: 34 x 66 blocks of 8x8-pixel tiles).
@@ -389,8 +394,8 @@ struct ListArgs {
   uint32_t* chunk_base;         // [chunks][32] entries per tile -> exclusive over the block's chunks
   unsigned long long* seg_look; // [segs][32] placing look-back words
   uint32_t* tile_base;          // [num_blocks][32] first entry of each tile
-  uint32_t* ranges;             // [tiles] (start, end), (0, 0) when empty
-  uint32_t* ids;                // [entry_cap] splat indices, tile by tile
+  uint32_t* ranges;             // [tiles] (first written entry, entries of the tile)
+  uint32_t* ids;                // [entry_cap] splat indices, up to kListLimit of every tile
   uint32_t entry_cap;
 };
 // Chunks, ballot groups and placing segments of a frame of at most pair_cap pairs.
@@ -552,6 +557,15 @@ struct CompositeArgs {
   FrameCounters* fc;
   uint32_t num_recs;        // splat records (ids at or above are rejected)
   uint32_t num_entries;     // sorted ids (ranges beyond are clamped)
+  // Screen-block lists (masks set): ranges hold (start, count) and sorted_ids
+  // the first kListLimit entries of each tile; the others come from the
+  // blocks' hit words.
+  const uint32_t* masks;
+  const uint32_t* chunk_base;
+  const uint32_t* chunk_first;
+  const uint32_t* block_start;
+  const uint32_t* sorted_pairs;
+  uint32_t blocks_x, num_blocks;
 };
 cudaError_t launch_composite(const CompositeArgs& a, cudaStream_t s);
 

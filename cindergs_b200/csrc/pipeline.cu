@@ -238,6 +238,8 @@ struct cgs_ctx {
   DevBuf lists, list_boxes;
   uint32_t list_pairs = 0, list_blocks = 0;
   uint32_t pair_cap = 0;        // pairs the buffers are wanted for
+  uint32_t list_cap = 0;        // entries of the tile lists that are wanted held
+  int list_src = 0;             // pair buffer holding the latest Stage 3's sorted pairs
   int pair_parity = 0;
   bool s3_lists = false;        // the latest Stage 3 went through the lists
   uint32_t entry_cap = 0;       // capacity of the key/id buffers (entries)
@@ -496,9 +498,30 @@ uint32_t cap_for(uint32_t count, uint32_t pct) {
                                       (uint64_t)kMaxEntryCap);
 }
 
+// Capacities after a frame with counters f: at least `pct` percent above what
+// it needed where that exceeds `share` percent of the current ones. A frame of
+// screen-block lists needs its pairs and the entries it held, one of the entry
+// sorts all its entries.
+void grow_caps(cgs_ctx* ctx, const FrameCounters& f, uint32_t share, uint32_t pct) {
+  auto grow = [&](uint32_t& cap, uint32_t need) {
+    if (need > (uint64_t)cap * share / 100) cap = std::max(cap, cap_for(need, pct));
+  };
+  if (f.pairs) {
+    grow(ctx->pair_cap, f.pairs);
+    grow(ctx->list_cap, f.written);
+  } else {
+    grow(ctx->entry_cap, f.entries);
+  }
+}
+
+// The frame did not fit the capacities it ran with.
+bool overflowed(const FrameCounters& f, uint32_t cap) {
+  return (f.status & kStatusCapacity) || (f.pairs ? f.written : f.entries) > cap;
+}
+
 // Buffers of d's Stage 3 at the context's current capacities.
 int ensure_stage3_buffers(cgs_ctx* ctx, const FrameDesc& d) {
-  if (d.lists) return ensure_list_buffers(ctx, ctx->entry_cap, ctx->pair_cap, d.num_blocks);
+  if (d.lists) return ensure_list_buffers(ctx, ctx->list_cap, ctx->pair_cap, d.num_blocks);
   return ensure_entry_buffers(ctx, ctx->entry_cap, d.key64, d.radix_bits);
 }
 
@@ -548,7 +571,7 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   a.chunk_base = (uint32_t*)(lp + B.base);
   a.ranges = ctx->ranges.as<uint32_t>();
   a.ids = ctx->ids[0].as<uint32_t>();
-  a.entry_cap = ctx->entry_cap;
+  a.entry_cap = ctx->list_cap;
   ctx->kbegin(CGS_K_BIN);
   CGS_CUDA(launch_list_pairs(a, s), "list pairs launch");
   ctx->kend();
@@ -574,6 +597,7 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   CGS_CUDA(run_radix_sort(so, &src, s), "pair sort");
   ctx->kend();
   a.sorted_pairs = (const uint32_t*)(lp + B.ids[src]);
+  ctx->list_src = src;
   ctx->kbegin(CGS_K_BIN);
   CGS_CUDA(launch_list_count(a, s), "list count launch");
   ctx->kend();
@@ -814,7 +838,19 @@ int enqueue_stage4(cgs_ctx* ctx, const FrameDesc& d, int result_src) {
   c.out_f32 = d.write_f32 ? ctx->fb_f32.as<float4>() : nullptr;
   c.fc = (FrameCounters*)sc;
   c.num_recs = d.max_n ? d.max_n : 1u;
-  c.num_entries = ctx->entry_cap;
+  c.num_entries = d.lists ? ctx->list_cap : ctx->entry_cap;
+  if (d.lists) {
+    const ScratchLayout L(d.n, d.max_n ? d.max_n : 1u);
+    const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+    const char* lp = ctx->lists.as<char>();
+    c.masks = (const uint32_t*)(lp + B.masks);
+    c.chunk_base = (const uint32_t*)(lp + B.base);
+    c.sorted_pairs = (const uint32_t*)(lp + B.ids[ctx->list_src]);
+    c.chunk_first = (const uint32_t*)(sc + L.lchunk);
+    c.block_start = (const uint32_t*)(sc + L.lstart);
+    c.blocks_x = d.blocks_x;
+    c.num_blocks = d.num_blocks;
+  }
   ctx->kbegin(CGS_K_COMPOSITE);
   CGS_CUDA(launch_composite(c, ctx->stream), "composite launch");
   ctx->kend();
@@ -830,8 +866,7 @@ int rerun_stage34(cgs_ctx* ctx) {
   const FrameCounters& f = ctx->h_ring[ctx->latest_slot].fc;
   // the entries are counted once all pairs are held: at most one run more
   for (int attempt = 0; attempt < 3; ++attempt) {
-    if (f.entries > ctx->entry_cap) ctx->entry_cap = cap_for(f.entries, 25);
-    if (d.lists && f.pairs > ctx->pair_cap) ctx->pair_cap = cap_for(f.pairs, 25);
+    grow_caps(ctx, f, 100, 25);
     CGS_TRY(ensure_stage3_buffers(ctx, d));
     // keep fc->surviving and fc->active (Stage 2's words); clear the Stage 3 words
     CGS_CUDA(cudaMemsetAsync(sc + 8, 0, sizeof(FrameCounters) - 8, ctx->stream), "clear counters");
@@ -879,7 +914,7 @@ int check_slot(cgs_ctx* ctx, int k, bool block) {
     ctx->sticky_msg = "a bounded device-side wait gave up during a frame";
   }
   if (status & kStatusPoisoned) ctx->poisoned = true;
-  if (p.stage3_ran && (status & kStatusCapacity || entries > p.cap)) {
+  if (p.stage3_ran && overflowed(h.fc, p.cap)) {
     if (k == ctx->latest_slot) {
       CGS_TRY(rerun_stage34(ctx));
       entries = ctx->h_ring[k].fc.entries;
@@ -887,13 +922,10 @@ int check_slot(cgs_ctx* ctx, int k, bool block) {
       // a later frame is in flight: its pixels are rendered again if a
       // readback waits for them (rerender_slot); the buffers grow now
       p.overflowed = true;
-      ctx->entry_cap = std::max(ctx->entry_cap, cap_for(entries, 30));
-      if (h.fc.pairs > ctx->pair_cap) ctx->pair_cap = cap_for(h.fc.pairs, 30);
+      grow_caps(ctx, h.fc, 100, 30);
     }
   } else if (p.stage3_ran) {
-    // keep 25% headroom for the next frames
-    if (entries > ctx->entry_cap / 10 * 8) ctx->entry_cap = cap_for(entries, 30);
-    if (h.fc.pairs > ctx->pair_cap / 10 * 8) ctx->pair_cap = cap_for(h.fc.pairs, 30);
+    grow_caps(ctx, h.fc, 80, 30);  // keep 25% headroom for the next frames
   }
   if (k == ctx->latest_slot) {
     if (p.stage3_ran) {
@@ -952,7 +984,7 @@ int check_slot(cgs_ctx* ctx, int k, bool block) {
         const uint64_t P = h.fc.pairs;
         kp.alg_bytes[CGS_K_BIN] += A * 8 + P * (8 + 4 + 48 + 4);
         kp.alg_bytes[CGS_K_ENTRY_SORT] +=
-            P * 16 * p.sort_passes + P * 8 + E * 4 + (uint64_t)p.total_tiles * 8;
+            P * 16 * p.sort_passes + P * 8 + (uint64_t)h.fc.written * 4 + (uint64_t)p.total_tiles * 8;
       } else {
         kp.alg_bytes[CGS_K_BIN] += A * 44 + E * (p.key64 ? 12 : 8);
       }
@@ -2182,6 +2214,9 @@ int enqueue_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_compositor* 
   if (!cached) {
     if (ctx->entry_cap == 0)
       ctx->entry_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(32ull * mn, 1u << 20), (uint64_t)kMaxEntryCap);
+    if (ctx->list_cap == 0)
+      ctx->list_cap = (uint32_t)std::min<uint64_t>((uint64_t)d.total_tiles * kListLimit,
+                                                   std::max<uint64_t>(32ull * mn, 1u << 20));
     if (ctx->pair_cap == 0)
       ctx->pair_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(4ull * mn, 1u << 16), (uint64_t)kMaxEntryCap);
     CGS_TRY(ensure_stage3_buffers(ctx, d));
@@ -2377,7 +2412,7 @@ int cgs_execute_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_composit
   P.split_possible = d.split_possible;
   P.key64 = d.key64;
   P.n = n;
-  P.cap = ctx->entry_cap;
+  P.cap = d.lists ? ctx->list_cap : ctx->entry_cap;
   P.lists = d.lists;
   P.sort_passes = passes;
   P.splat_passes = splat_passes;
@@ -2452,22 +2487,18 @@ namespace {
 // listed (the capacity is grown for them and kept 30% above the largest
 // count).
 int check_views(cgs_ctx* ctx, uint32_t nv, const uint32_t* cap_used,
-                std::vector<uint32_t>* overflowed, uint64_t* total_entries) {
-  uint32_t most = 0, pairs = 0;
+                std::vector<uint32_t>* overflowed_views, uint64_t* total_entries) {
   *total_entries = 0;
-  overflowed->clear();
+  overflowed_views->clear();
   for (uint32_t v = 0; v < nv; ++v) {
     const FrameCounters& fc = ctx->h_views[v].fc;
     if (fc.status & kStatusPoisoned) ctx->poisoned = true;
     if (fc.status & (kStatusLookbackTimeout | kStatusBarrierTimeout))
       return ctx->fail(CGS_E_TIMEOUT, "a bounded device-side wait gave up during a view");
-    if ((fc.status & kStatusCapacity) || fc.entries > cap_used[v]) overflowed->push_back(v);
-    most = std::max(most, fc.entries);
-    pairs = std::max(pairs, fc.pairs);
+    if (overflowed(fc, cap_used[v])) overflowed_views->push_back(v);
     *total_entries += fc.entries;
   }
-  if (most > ctx->entry_cap / 10 * 8) ctx->entry_cap = cap_for(most, 30);
-  if (pairs > ctx->pair_cap / 10 * 8) ctx->pair_cap = cap_for(pairs, 30);
+  for (uint32_t v = 0; v < nv; ++v) grow_caps(ctx, ctx->h_views[v].fc, 80, 30);
   return CGS_OK;
 }
 
@@ -2482,7 +2513,7 @@ int enqueue_view(cgs_ctx* ctx, const cgs_camera* cam, const cgs_compositor* comp
   ctl.out_pitch = comp->screen_width ? comp->screen_width : 1u;
   FrameInfo fi;
   CGS_TRY(enqueue_frame(ctx, cam, comp, params, ctl, &fi));
-  *cap_used = ctx->entry_cap;
+  *cap_used = fi.d.lists ? ctx->list_cap : ctx->entry_cap;
   return CGS_OK;
 }
 
@@ -2628,6 +2659,7 @@ int cgs_execute_views(cgs_ctx* ctx, uint32_t num_views, const cgs_camera* camera
     put_bytes(k, &ctx->state_epoch, sizeof(ctx->state_epoch));
     put_bytes(k, &ctx->entry_cap, sizeof(ctx->entry_cap));
     put_bytes(k, &ctx->pair_cap, sizeof(ctx->pair_cap));
+    put_bytes(k, &ctx->list_cap, sizeof(ctx->list_cap));
     return k;
   };
   CGS_CUDA(cudaEventRecord(ctx->views_ev[0], s), "views event");
@@ -2639,8 +2671,10 @@ int cgs_execute_views(cgs_ctx* ctx, uint32_t num_views, const cgs_camera* camera
     ctx->splat_parity = ctx->views_splat_parity;
     ctx->pair_parity = ctx->views_pair_parity;
     st.graph_replayed = 1;
-    std::vector<uint32_t> cap(num_views, ctx->entry_cap), over;
-    const uint32_t cap_before = ctx->entry_cap, pairs_before = ctx->pair_cap;
+    std::vector<uint32_t> cap(num_views), over;
+    for (uint32_t v = 0; v < num_views; ++v)
+      cap[v] = ctx->h_views[v].fc.pairs ? ctx->list_cap : ctx->entry_cap;
+    const uint32_t cap_before = ctx->entry_cap, pairs_before = ctx->pair_cap, list_before = ctx->list_cap;
     CGS_TRY(check_views(ctx, num_views, cap.data(), &over, &st.total_tile_entries));
     for (int round = 0; !over.empty() && round < 3; ++round) {
       // render the overflowed views again eagerly; the graph is rebuilt on
@@ -2653,7 +2687,8 @@ int cgs_execute_views(cgs_ctx* ctx, uint32_t num_views, const cgs_camera* camera
       CGS_TRY(check_views(ctx, num_views, cap.data(), &over, &st.total_tile_entries));
     }
     if (!over.empty()) return ctx->fail(CGS_E_CAPACITY, "tile entries exceeded the key buffers");
-    if (ctx->entry_cap != cap_before || ctx->pair_cap != pairs_before) drop_views_graph(ctx);
+    if (ctx->entry_cap != cap_before || ctx->pair_cap != pairs_before || ctx->list_cap != list_before)
+      drop_views_graph(ctx);
   } else {
     CGS_TRY(views_eager(ctx, num_views, cameras, comps, prm.data(), d_rgba8, &st.views_rerendered,
                         &st.total_tile_entries));
@@ -2763,9 +2798,8 @@ int rerender_slot(cgs_ctx* ctx, int k, uint32_t* out, uint32_t pitch) {
       rc = ctx->fail(CGS_E_TIMEOUT, "a bounded device-side wait gave up during a re-render");
       break;
     }
-    if (!(f.status & kStatusCapacity) && f.entries <= ctx->entry_cap) break;
-    if (f.entries > ctx->entry_cap) ctx->entry_cap = cap_for(f.entries, 30);
-    if (f.pairs > ctx->pair_cap) ctx->pair_cap = cap_for(f.pairs, 30);
+    if (!overflowed(f, fi.d.lists ? ctx->list_cap : ctx->entry_cap)) break;
+    grow_caps(ctx, f, 100, 30);
     rc = ctx->fail(CGS_E_CAPACITY, "tile entries exceed the largest key buffers");
   }
   ctx->kprof = kp;
@@ -2932,26 +2966,58 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
     cudaError_t e = cudaMemcpy(tmp.data(), b.p, bytes, cudaMemcpyDeviceToHost);
     return e == cudaSuccess ? CGS_OK : ctx->cuda_fail(e, "buffer readback");
   };
-  // screen-block lists: the splat indices in tile order and the tiles' ranges
+  // screen-block lists: the splat indices in tile order and the tiles' ranges,
+  // from the blocks' hit words
   std::vector<uint32_t> l_ids, l_ranges;
   auto fetch_lists = [&]() -> int {
-    const size_t tiles = ctx->last_tiles;
-    CGS_TRY(fetch(ctx->ranges, tiles * 8));
-    std::vector<uint32_t> r(2 * tiles);
-    std::memcpy(r.data(), tmp.data(), tiles * 8);
-    CGS_TRY(fetch(ctx->ids[ctx->s3_src], entries * 4));
-    const uint32_t* in = (const uint32_t*)tmp.data();
-    l_ids.reserve(entries);
-    l_ranges.assign(2 * tiles, 0);
-    for (size_t t = 0; t < tiles; ++t) {
-      const uint32_t a = r[2 * t], b = r[2 * t + 1];
-      if (a >= b) continue;
-      if (b > entries || l_ids.size() + (b - a) > entries)
-        return ctx->fail(CGS_E_STATE, "tile range out of bounds");
-      l_ranges[2 * t] = (uint32_t)l_ids.size();
-      l_ids.insert(l_ids.end(), in + a, in + b);
-      l_ranges[2 * t + 1] = (uint32_t)l_ids.size();
+    const FrameDesc& d = ctx->last_desc;
+    const ScratchLayout L(d.n, d.max_n ? d.max_n : 1u);
+    const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+    auto words = [&](const DevBuf& buf, size_t off, size_t n, std::vector<uint32_t>* out) -> int {
+      out->resize(n);
+      if (n == 0) return CGS_OK;
+      if (!buf.p || buf.cap < off + n * 4) return ctx->fail(CGS_E_STATE, "buffer not populated by the last frame");
+      const cudaError_t e = cudaMemcpy(out->data(), buf.as<char>() + off, n * 4, cudaMemcpyDeviceToHost);
+      return e == cudaSuccess ? CGS_OK : ctx->cuda_fail(e, "buffer readback");
+    };
+    std::vector<uint32_t> start, chunk, masks, pairs;
+    CGS_TRY(words(ctx->scratch, L.lstart, d.num_blocks + 1, &start));
+    CGS_TRY(words(ctx->scratch, L.lchunk, d.num_blocks + 1, &chunk));
+    const uint32_t np = start[d.num_blocks], groups = np <= kListSmallPairs ? 1u : kListGroups;
+    CGS_TRY(words(ctx->lists, B.masks, (size_t)chunk[d.num_blocks] * groups * 32, &masks));
+    CGS_TRY(words(ctx->lists, B.ids[ctx->list_src], np, &pairs));
+    // every (tile, first pair, word) in block and pair order, twice: counts, then places
+    std::vector<uint32_t> at(d.total_tiles, 0);
+    auto walk = [&](auto&& fn) {
+      for (uint32_t b = 0; b < d.num_blocks; ++b)
+        for (uint32_t k = 0; k < (chunk[b + 1] - chunk[b]) * groups; ++k) {
+          const uint32_t i0 = start[b] + 32 * k;
+          if (i0 >= start[b + 1]) continue;
+          for (uint32_t t = 0; t < 32; ++t) {
+            const uint32_t tx = ((b % d.blocks_x) << kListBlockW) + (t & 7u);
+            const uint32_t ty = ((b / d.blocks_x) << kListBlockH) + (t >> 3);
+            const uint32_t m = masks[((size_t)chunk[b] * groups + k) * 32 + t];
+            if (m && tx < d.tiles_x && ty < d.tiles_y) fn(ty * d.tiles_x + tx, i0, m);
+          }
+        }
+    };
+    walk([&](uint32_t tile, uint32_t, uint32_t m) { at[tile] += (uint32_t)__builtin_popcount(m); });
+    l_ranges.assign(2 * (size_t)d.total_tiles, 0);
+    uint32_t run = 0;
+    for (uint32_t t = 0; t < d.total_tiles; ++t) {
+      if (at[t]) {
+        l_ranges[2 * (size_t)t] = run;
+        l_ranges[2 * (size_t)t + 1] = run + at[t];
+      }
+      const uint32_t n = at[t];
+      at[t] = run;
+      run += n;
     }
+    if (run != entries) return ctx->fail(CGS_E_STATE, "the lists' words and the entry total differ");
+    l_ids.resize(run);
+    walk([&](uint32_t tile, uint32_t i0, uint32_t m) {
+      for (; m; m &= m - 1) l_ids[at[tile]++] = pairs[i0 + (uint32_t)__builtin_ctz(m)];
+    });
     return CGS_OK;
   };
   auto bytes_of = [](const std::vector<uint32_t>& v) {

@@ -16,8 +16,10 @@
 //                 row) and transposes the 32 words: tile t's word is its list
 //                 of these 32 splats, already in depth order;
 //   k_list_place: each chunk's first entry per tile inside its block, the
-//                 tiles' first entries and their [start, end) ranges;
-//   k_list_write: every word's splats are stored at their places.
+//                 tiles' first entries and counts;
+//   k_list_write: the words' splats are stored at their places, the front-most
+//                 1,024 of every tile (the compositor takes the rest from the
+//                 words, if it ever gets there).
 //
 // An entry costs one bit and one 4-byte store instead of a 4-byte key
 // and a 4-byte index written by the binning and moved by two or three radix
@@ -287,8 +289,8 @@ __global__ void __launch_bounds__(kListThreads) k_list_count(const ListArgs a) {
 // sums go through a look-back over the block's earlier segments (vectors of 32
 // words), and its chunks' counts become exclusive sums over the block's
 // chunks. The block's last segment knows the tiles' totals: it takes the
-// block's entries from a counter and writes the tiles' first entries and
-// ranges. 32 tiles x 8 parts of 8 chunks.
+// block's places from a counter and writes the tiles' first entries and
+// counts. 32 tiles x 8 parts of 8 chunks.
 __global__ void __launch_bounds__(256) k_list_place(const ListArgs a) {
   __shared__ uint32_t s_part[8][32];
   __shared__ uint32_t s_excl[32];
@@ -345,26 +347,34 @@ __global__ void __launch_bounds__(256) k_list_place(const ListArgs a) {
       s_excl[t] = excl;
       __syncwarp();
       if (seg + 1 == s1) {
-        const uint32_t n = excl + agg;  // the tile's entries
-        unsigned long long incl = n;
+        const uint32_t n = excl + agg;  // the tile's entries, the first `held` of them written
+        const uint32_t held = min(n, kListLimit);
+        unsigned long long all = n;
+        uint32_t incl = held;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-          const unsigned long long y = __shfl_up_sync(0xffffffffu, incl, o);
-          if (t >= (uint32_t)o) incl += y;
+          const unsigned long long y = __shfl_up_sync(0xffffffffu, all, o);
+          const uint32_t z = __shfl_up_sync(0xffffffffu, incl, o);
+          if (t >= (uint32_t)o) {
+            all += y;
+            incl += z;
+          }
         }
-        unsigned long long at = 0;
-        const unsigned long long cap = a.entry_cap;
+        // at most 32 x kListLimit entries in each of kListMaxBlocks blocks
+        static_assert((unsigned long long)kListLimit * 32 * kListMaxBlocks < (1ull << 32), "32-bit places");
+        uint32_t at = 0;
+        const uint32_t cap = a.entry_cap;
         if (t == 31) {
-          at = incl ? atomicAdd(&a.fc->stage_ctr, incl) : 0ull;
+          if (all) atomicAdd(&a.fc->stage_ctr, all);
+          at = incl ? atomicAdd(&a.fc->written, incl) : 0u;
           if (at + incl > cap) atomicOr(&a.fc->status, kStatusCapacity);
         }
-        at = __shfl_sync(0xffffffffu, at, 31) + incl - n;
-        a.tile_base[(size_t)b * 32 + t] = (uint32_t)min(at, cap);  // at the capacity: not written
+        at = __shfl_sync(0xffffffffu, at, 31) + incl - held;
+        a.tile_base[(size_t)b * 32 + t] = min(at, cap);  // at the capacity: not written
         const uint32_t tx = ((b % a.blocks_x) << kListBlockW) + (t & 7u);
         const uint32_t ty = ((b / a.blocks_x) << kListBlockH) + (t >> 3);
         if (tx < a.tiles_x && ty < a.tiles_y)
-          reinterpret_cast<uint2*>(a.ranges)[(size_t)ty * a.tiles_x + tx] =
-              n ? make_uint2((uint32_t)min(at, cap), (uint32_t)min(at + n, cap)) : make_uint2(0u, 0u);
+          reinterpret_cast<uint2*>(a.ranges)[(size_t)ty * a.tiles_x + tx] = make_uint2(min(at, cap), n);
       }
     }
     __syncthreads();
@@ -379,31 +389,36 @@ __global__ void __launch_bounds__(256) k_list_place(const ListArgs a) {
   }
 }
 
-// Entries. A warp takes two groups of 32 pairs at a time: lane t walks the set
-// bits of tile t's two ballots and lists them in shared memory, tile after
-// tile; then the warp copies that list out, one entry per lane, so that a
-// tile's entries of the 64 pairs (about 14 at 1080p) are stored together.
+// Entries, the first kListLimit of every tile. A warp takes two groups of 32
+// pairs at a time: lane t walks the set bits of tile t's two words and lists
+// them in shared memory, tile after tile; then the warp copies that list out,
+// one entry per lane, so that a tile's entries of the 64 pairs (about 14 at
+// 1080p) are stored together. Chunks whose tiles all have their kListLimit
+// entries are passed over: at 26M entries 72 -> 22 us.
 __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
   __shared__ uint16_t s_stage[kListWarps][64 * 32];  // tile << 6 | pair
   __shared__ uint32_t s_sid[kListWarps][64];
-  __shared__ uint32_t s_delta[kListWarps][32];
+  __shared__ uint32_t s_delta[kListWarps][32], s_end[kListWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunks = a.plan->chunks, groups = a.plan->groups;
-  const uint32_t cap = a.entry_cap;
   if (blockIdx.x == 0 && threadIdx.x == 0)
     a.fc->entries = (uint32_t)min(a.fc->stage_ctr, 0xFFFFFFFFull);
   uint16_t* stage = s_stage[warp];
   for (uint32_t c = blockIdx.x * kListWarps + warp; c < chunks; c += gridDim.x * kListWarps) {
+    uint32_t rank = a.chunk_base[(size_t)c * 32 + lane];
+    if (!__any_sync(0xffffffffu, rank < kListLimit)) continue;
     const uint32_t b = block_of(a.chunk_first, a.num_blocks, c);
     const uint32_t i0 = a.block_start[b] + (c - a.chunk_first[b]) * 32u * groups;
     const uint32_t end = min(a.block_start[b + 1], a.pair_cap);
-    uint64_t at = (uint64_t)a.tile_base[(size_t)b * 32 + lane] + a.chunk_base[(size_t)c * 32 + lane];
-    uint32_t p = (uint32_t)min(at, (uint64_t)cap);  // at the capacity: not written
+    const uint32_t first = a.tile_base[(size_t)b * 32 + lane];
+    s_end[warp][lane] = min(first + kListLimit, a.entry_cap);
     for (uint32_t j = 0; j < groups && i0 + 32u * j < end; j += 2) {
       const uint32_t i = i0 + 32u * j + lane;
       const bool two = j + 1 < groups && i0 + 32u * (j + 1) < end;
+      const bool on = rank < kListLimit;
+      if (!__any_sync(0xffffffffu, on)) break;
       const uint32_t* in = a.masks + ((size_t)c * groups + j) * 32 + lane;
-      const uint32_t m0 = in[0], m1 = two ? in[32] : 0u;
+      const uint32_t m0 = on ? in[0] : 0u, m1 = on && two ? in[32] : 0u;
       s_sid[warp][lane] = i < end ? a.sorted_pairs[i] : 0u;
       if (two) s_sid[warp][lane + 32] = i + 32 < end ? a.sorted_pairs[i + 32] : 0u;
       const uint32_t n = __popc(m0) + __popc(m1);
@@ -414,7 +429,7 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
         if (lane >= o) incl += y;
       }
       const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-      s_delta[warp][lane] = p - (incl - n);
+      s_delta[warp][lane] = first + rank - (incl - n);
       // from the highest bit down, backwards from the tile's end
       uint16_t* at_s = stage + incl;
       const uint32_t tile = (uint32_t)lane << 6;
@@ -430,13 +445,14 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
       }
       __syncwarp();
       for (uint32_t k = lane; k < total; k += 32) {
-        const uint32_t e = stage[k];
-        const uint32_t pos = s_delta[warp][e >> 6] + k;
-        if (pos < cap) a.ids[pos] = s_sid[warp][e & 63u];
+        const uint32_t e = stage[k], t = e >> 6;
+        const uint32_t pos = s_delta[warp][t] + k;
+        if (pos < s_end[warp][t]) a.ids[pos] = s_sid[warp][e & 63u];
       }
-      p = min(p + n, cap);
+      rank += n;
       __syncwarp();
     }
+    __syncwarp();
   }
 }
 

@@ -118,6 +118,49 @@ __device__ __forceinline__ uint32_t block_mask(const float4 geo, const float4 cc
   return m;
 }
 
+// Splats of entries [r0, r1) of tile (tx, ty), past those that the lists hold:
+// from the hit words of the tile's screen block (stage3_lists.cu), a group of
+// 32 pairs per thread and step. *cur is the chunk to start from (0 at first: a
+// search over the chunks' exclusive counts); the steps go on from the chunk
+// where the last entries were found. Called by the whole block.
+__device__ __forceinline__ void ids_beyond(const CompositeArgs& a, uint32_t tx, uint32_t ty, uint32_t r0,
+                                        uint32_t r1, uint32_t* cur, uint32_t* s_ids, uint32_t* s_red) {
+  const uint32_t blk = (ty >> kListBlockH) * a.blocks_x + (tx >> kListBlockW);
+  const uint32_t t = ((ty & ((1u << kListBlockH) - 1u)) << kListBlockW) | (tx & ((1u << kListBlockW) - 1u));
+  const uint32_t groups = a.block_start[a.num_blocks] <= kListSmallPairs ? 1u : kListGroups;
+  const uint32_t c0 = a.chunk_first[blk], c1 = a.chunk_first[blk + 1];
+  const uint32_t p0 = a.block_start[blk], p1 = a.block_start[blk + 1];
+  uint32_t c = *cur;
+  if (c < c0) {
+    uint32_t lo = c0, hi = c1;  // base[lo] <= r0
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (a.chunk_base[(size_t)mid * 32 + t] <= r0)
+        lo = mid;
+      else
+        hi = mid;
+    }
+    c = lo;
+  }
+  for (uint32_t k = threadIdx.x; k < r1 - r0; k += blockDim.x) s_ids[k] = kInvalid;
+  while (c < c1) {
+    const uint32_t g = threadIdx.x % groups, ci = c + threadIdx.x / groups;
+    const uint32_t i0 = p0 + (ci - c0) * 32u * groups + 32u * g;
+    uint32_t m = 0;
+    if (ci < c1 && i0 < p1) m = a.masks[((size_t)ci * groups + g) * 32 + t];
+    uint32_t total;
+    uint32_t rank = a.chunk_base[(size_t)c * 32 + t];
+    const uint32_t first = rank;
+    rank += block_exclusive_sum(__popc(m), s_red, &total);
+    for (; m; m &= m - 1u, ++rank)
+      if (rank >= r0 && rank < r1) s_ids[rank - r0] = a.sorted_pairs[i0 + (uint32_t)__ffs(m) - 1u];
+    if (first + total >= r1) break;
+    c += blockDim.x / groups;
+  }
+  *cur = c;
+  __syncthreads();
+}
+
 template <int LW, int LH>
 __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArgs a) {
   constexpr uint32_t TW = 1u << LW, TH = 1u << LH, kCompThreads = TW * TH;
@@ -126,16 +169,24 @@ __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArg
   // [kBatch]: a record of opacity 0 that fills up a group of four
   __shared__ __align__(128) SplatRec s_rec[2][kBatch + 1];
   __shared__ uint32_t s_bits[kBatch / 32][NW];  // entries of a batch per warp
+  __shared__ uint32_t s_ids[kBatch], s_red[32];  // entries beyond the lists
+  static_assert(kListLimit % kBatch == 0, "a batch is in the lists or beyond them");
 
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   const uint32_t tile_id = blockIdx.x, tx = tile_id % a.tiles_x, ty = tile_id / a.tiles_x;
   const uint32_t px = tx * TW + (warp % BX) * 8u + (lane & 7u);
   const uint32_t py = ty * TH + (warp / BX) * 4u + (lane >> 3);
   const bool inside = px < a.width && py < a.height;
-  const uint32_t rs = min(a.ranges[2 * (size_t)tile_id], a.num_entries);
-  const uint32_t re = min(a.ranges[2 * (size_t)tile_id + 1], a.num_entries);
-  const bool empty = rs >= re;
-  const uint32_t n = empty ? 0u : re - rs;
+  const bool lists = a.masks != nullptr;
+  const uint2 range = reinterpret_cast<const uint2*>(a.ranges)[tile_id];
+  const uint32_t rs = min(range.x, a.num_entries);
+  const uint32_t re = min(range.y, a.num_entries);
+  // what overflowed the entry buffer (flagged, rendered again) is left out
+  const uint32_t n = !lists ? re - min(rs, re)
+                     : a.num_entries - rs < min(range.y, kListLimit) ? a.num_entries - rs : range.y;
+  const uint32_t beyond = lists ? kListLimit / kBatch : 0xFFFFFFFFu;  // first batch past the lists
+  const bool empty = n == 0u;
+  uint32_t cur = 0;  // chunk of the entries beyond the lists
   const uint32_t nb = (n + kBatch - 1) / kBatch;
 
   auto issue = [&](uint32_t b) {
@@ -143,7 +194,7 @@ __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArg
     const uint32_t cnt = min((uint32_t)kBatch, n - b * kBatch);
     for (uint32_t c = tid; c < cnt * 3u; c += kCompThreads) {
       const uint32_t k = c / 3u, part = c - 3u * k;
-      uint32_t id = a.sorted_ids[rs + b * kBatch + k];
+      uint32_t id = b >= beyond ? s_ids[k] : a.sorted_ids[rs + b * kBatch + k];
       if (id >= a.num_recs) {  // never let a bad id become an out-of-bounds copy
         if (a.fc) atomicOr(&a.fc->status, kStatusCapacity);
         id = 0;
@@ -173,6 +224,8 @@ __global__ void __launch_bounds__(1 << (LW + LH)) k_composite(const CompositeArg
   for (uint32_t b = 0; b < nb; ++b) {
     const uint32_t stage = b & 1u;
     if (b + 1 < nb) {
+      if (b + 1 >= beyond)
+        ids_beyond(a, tx, ty, (b + 1) * kBatch, min((b + 2) * kBatch, n), &cur, s_ids, s_red);
       issue(b + 1);
       issued = b + 2;
     }

@@ -38,6 +38,31 @@ def test_block_edges(n, wh):
         st.close()
 
 
+# faint splats: lists of thousands of entries that no pixel saturates before,
+# so the compositor goes past the 1,024 written ones (one group and four
+# groups per chunk, blocks of 64, 256 and 512 threads)
+@pytest.mark.parametrize("n,wh,shape,grow", [(6_000, (64, 48), _abi.TILE_16X16, 40.0),
+                                             (60_000, (200, 130), _abi.TILE_32X16, 4.0),
+                                             (60_000, (100, 70), _abi.TILE_8X8, 20.0),
+                                             (90_000, (300, 200), _abi.TILE_16X16, 4.0)])
+def test_beyond_the_written_entries(n, wh, shape, grow):
+    st = GpuPipelineState(0)
+    try:
+        scene = random_scene(n, seed=9)
+        scene.covariances_3d[:] *= np.float32(grow)
+        scene.opacities[:] = np.random.default_rng(1).uniform(0.0042, 0.008, n).astype(np.float32)
+        st.upload_scene(scene)
+        t, g, cam, comp = run(st, scene, *wh, tile_shape=shape)
+        o = oracle_frame(scene, cam, comp, tile=_abi.TILE_SHAPES[shape])
+        assert int((g["ranges"][1::2] - g["ranges"][0::2]).max()) > 2048
+        assert_stage23_exact(g, o)
+        assert np.abs(g["f32"] - o["rgba_f32"]).max() <= 2e-3
+        _, r, _, _ = run(st, scene, *wh, tile_shape=shape, entry_sort=_abi.SORT_RADIX)
+        np.testing.assert_array_equal(g["f32"], r["f32"])
+    finally:
+        st.close()
+
+
 # (n, viewport, tile shape, covariance scale): more than 2^18 pairs (four groups
 # per chunk), two pair-sort passes (460 and 1,020 blocks), splats over whole
 # screens (the pair buffers overflow on the first frame), 64-bit keys

@@ -347,8 +347,10 @@ __global__ void __launch_bounds__(256) k_field_update(FieldUpdate a) {
   else
     gi = a.g[i];
   if (!a.adam) return;
-  const float mi = a.b1 * a.m[i] + (1.0f - a.b1) * gi;
-  const float vi = a.b2 * a.v[i] + (1.0f - a.b2) * gi * gi;
+  // one rounding order of the moments, written out: left to the compiler, it
+  // moved with the code around it, and the optimiser carries each last bit on
+  const float mi = __fmaf_rn(1.0f - a.b1, gi, __fmul_rn(a.b1, a.m[i]));
+  const float vi = __fmaf_rn(__fmul_rn(1.0f - a.b2, gi), gi, __fmul_rn(a.b2, a.v[i]));
   a.m[i] = mi;
   a.v[i] = vi;
   const float pi = a.p[i] - a.lr * (mi * a.c1) / (sqrtf(vi * a.c2) + a.eps);

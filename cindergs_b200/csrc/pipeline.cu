@@ -1498,9 +1498,10 @@ int mvc_bind(cgs_ctx* ctx, bool learned, float threshold, bool cache, uint32_t* 
     const size_t scan_status = ((size_t)scan_tiles(n) + 1) * 8 + 64;
     CGS_CUDA(cudaMalloc(&flag.p, (size_t)n * 4), "mvc flags");
     flag.cap = (size_t)n * 4;
-    CGS_CUDA(cudaMalloc(&slot.p, (size_t)n * 4 + scan_status), "mvc slots");
-    slot.cap = (size_t)n * 4 + scan_status;
-    char* sb = slot.as<char>() + (size_t)n * 4;
+    const size_t slot_bytes = ((size_t)n * 4 + 7) & ~(size_t)7;  // 64-bit scan words follow
+    CGS_CUDA(cudaMalloc(&slot.p, slot_bytes + scan_status), "mvc slots");
+    slot.cap = slot_bytes + scan_status;
+    char* sb = slot.as<char>() + slot_bytes;
     uint32_t* words = (uint32_t*)(sb + scan_status - 64);
     uint32_t hw[4] = {};
     int rc = CGS_OK;

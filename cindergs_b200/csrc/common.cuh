@@ -87,6 +87,18 @@ __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
   return v;
 }
 
+// Programmatic dependent launches (launch_dependent in kernels.h): a kernel
+// lets the next one of the stream start its blocks once all of its own have
+// started, and waits, before it touches anything an earlier kernel writes or
+// reads, until that one has completed. Both do nothing in a kernel launched
+// the usual way.
+__device__ __forceinline__ void dependents_may_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void wait_for_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Block-wide exclusive sum over one u32 per thread (blockDim.x a multiple of
 // 32, at most 1024). `warp_sums` is shared scratch of 32 words. Returns the
 // exclusive prefix; *total receives the block sum.

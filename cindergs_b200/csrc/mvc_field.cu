@@ -85,6 +85,8 @@ constexpr int kGatherRows = 32;
 __global__ void __launch_bounds__(256) k_field_gather(FieldBatch fb) {
   __shared__ float xh[kGatherRows][3];
   __shared__ __nv_bfloat16 tile[kIn][kGatherRows + 2];
+  dependents_may_start();
+  wait_for_previous_kernel();
   const uint32_t r0 = blockIdx.x * kGatherRows;
   if (threadIdx.x < kGatherRows) {
     const uint32_t r = r0 + threadIdx.x;
@@ -212,6 +214,8 @@ __global__ void __launch_bounds__(32 * kLossRows, 1) k_field_loss(FieldLoss fl) 
   __shared__ float s_loss[2][kLossRows];
   const uint32_t V = fl.V, row0 = blockIdx.x * kLossRows;
   const uint32_t lane = threadIdx.x & 31u, q = threadIdx.x >> 5, row = row0 + q;
+  dependents_may_start();
+  wait_for_previous_kernel();
   for (uint32_t j = threadIdx.x; j < V; j += 32 * kLossRows) sv[j] = fl.verts[j];
   const bool on = row < fl.B;
   const float* z = fl.z + (size_t)(on ? row : 0u) * fl.ldz;
@@ -325,6 +329,8 @@ __global__ void __launch_bounds__(32 * kLossRows, 1) k_field_loss(FieldLoss fl) 
 // (1-b2) g^2; p -= lr mh / (sqrt(vh) + eps) with the bias corrections mh = m
 // c1, vh = v c2; refreshes the bf16 copy and the transposed weights.
 __global__ void __launch_bounds__(256) k_field_update(FieldUpdate a) {
+  dependents_may_start();
+  wait_for_previous_kernel();
   const uint32_t i = blockIdx.x * 256 + threadIdx.x;
   if (i >= a.off[10]) return;
   float gi = 0.0f;
@@ -711,8 +717,7 @@ __global__ void __launch_bounds__(kApWarps * 32, 1) k_field_apply(FieldInfer fi)
 
 cudaError_t launch_field_gather(const FieldBatch& b, cudaStream_t s) {
   if (b.B == 0) return cudaSuccess;
-  k_field_gather<<<(b.B + kGatherRows - 1) / kGatherRows, 256, 0, s>>>(b);
-  return cudaGetLastError();
+  return launch_dependent(k_field_gather, (b.B + kGatherRows - 1) / kGatherRows, 256, 0, s, b);
 }
 
 cudaError_t launch_field_refresh(const uint32_t* off, uint32_t V, uint32_t ldV, const float* p,
@@ -738,8 +743,7 @@ cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s) {
           cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    kernel<<<(l.B + kLossRows - 1) / kLossRows, 32 * kLossRows, smem, s>>>(l);
-    return cudaGetLastError();
+    return launch_dependent(kernel, (l.B + kLossRows - 1) / kLossRows, 32 * kLossRows, smem, s, l);
   };
   if (l.V <= 192u) return run(k_field_loss<6>);
   if (l.V <= 672u) return run(k_field_loss<21>);
@@ -747,8 +751,7 @@ cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s) {
 }
 
 cudaError_t launch_field_update(const FieldUpdate& u, cudaStream_t s) {
-  k_field_update<<<(u.off[10] + 255) / 256, 256, 0, s>>>(u);
-  return cudaGetLastError();
+  return launch_dependent(k_field_update, (u.off[10] + 255) / 256, 256, 0, s, u);
 }
 
 cudaError_t launch_field_project(const FieldNet& net, uint32_t V, const float4* rest,

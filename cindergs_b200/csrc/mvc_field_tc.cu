@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kTcWG * 128, 1) k_field_infer_tc(FieldInfer fi
 // = 32 puts 128 CTAs on a layer instead of 32 (16 us a layer with NT = 128).
 constexpr uint32_t kGmTile = 128, kGmBK = 64;
 constexpr int kGmThreads = 256;
-constexpr uint32_t kGmSumRows = 64, kGmSumStages = 8;  // column-sum ring
+constexpr uint32_t kGmSumRows = 128, kGmSumStages = 4;  // column-sum ring
 __host__ __device__ constexpr uint32_t gm_stage_bytes(uint32_t nt) { return (kGmTile + nt) * kGmBK * 2; }
 // dynamic shared memory of `stages` stages, rounded so that the barriers follow
 __host__ __device__ constexpr uint32_t gm_smem(uint32_t nt, uint32_t stages) {
@@ -579,6 +579,11 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& g, uint32_t m0, uint32
   const uint32_t tmem = *s_tmem;
   const uint32_t base = smem_u32(sm);
   const uint32_t idesc = idesc_bf16(kGmTile, NT, 0, 0);
+  // Only now that this block holds its tensor memory may blocks of the next
+  // kernel, which allocate theirs, become its neighbours: one that came first
+  // could keep the columns this one needs while it waits for this kernel.
+  dependents_may_start();
+  wait_for_previous_kernel();  // the set-up above overlaps it
 
   // block kb of A rows m0.. and B rows n0.. into stage kb % stages
   auto load = [&](uint32_t kb) {
@@ -792,6 +797,8 @@ __device__ __forceinline__ void column_sums(const float* in, uint32_t B, uint32_
 __global__ void __launch_bounds__(kGmThreads) k_gemm_grads(GemmBatch b, uint32_t sum_blocks) {
   uint32_t i = blockIdx.x;
   if (i < sum_blocks) {
+    dependents_may_start();
+    wait_for_previous_kernel();
 #pragma unroll 1
     for (int p = 0; p < kGradProblems; ++p) {
       const uint32_t nb = (b.sum_n[p] + 31) / 32;
@@ -848,8 +855,7 @@ cudaError_t launch_gemm_nt(const GemmArgs& g, int epi, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const uint32_t stages = std::min((g.K + kGmBK - 1) / kGmBK, 2 * A);
     const dim3 grid((g.N + nt - 1) / nt, (g.M + kGmTile - 1) / kGmTile);
-    kernel<<<grid, kGmThreads, gm_smem(nt, stages), s>>>(g);
-    return cudaGetLastError();
+    return launch_dependent(kernel, grid, kGmThreads, gm_smem(nt, stages), s, g);
   };
   if (epi == kEpiBias) return run(k_gemm_tc<kEpiBias, 64, 2>, 64, 2);
   if (epi == kEpiBiasSilu) return run(k_gemm_tc<kEpiBiasSilu, 32, 2>, 32, 2);
@@ -879,8 +885,7 @@ cudaError_t launch_gemm_grads(const GemmBatch& b, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   uint32_t sums = 0;
   for (int p = 0; p < kGradProblems; ++p) sums += (b.sum_n[p] + 31) / 32;
-  k_gemm_grads<<<sums + b.first[kGradProblems] * b.splits, kGmThreads, smem, s>>>(b, sums);
-  return cudaGetLastError();
+  return launch_dependent(k_gemm_grads, sums + b.first[kGradProblems] * b.splits, kGmThreads, smem, s, b, sums);
 }
 
 }  // namespace cgs

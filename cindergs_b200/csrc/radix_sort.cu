@@ -24,6 +24,9 @@
 // does the same for standalone sorts); k_digit_bases turns them into
 // exclusive bases once per sort. HBM traffic per pass: one read and one write
 // of keys and payloads (16 B per pair), plus 1 KiB of look-back words per tile.
+// The passes are dependent launches: a pass's blocks start while the one before
+// it drains and wait before their first access (3M pairs, 4 passes with the
+// histogram: 194 -> 183 us; a frame's splat and pair sorts: 7 to 9 us less).
 #include "kernels.h"
 
 namespace cgs {
@@ -156,6 +159,8 @@ __global__ void __launch_bounds__(kSortThreads, PAY2 ? 3 : 4) k_onesweep(const P
   uint32_t* s_misc = s_goff + R;                 // [40]: tile, warp sums
   uint32_t* s_wor = s_misc + 48;                 // [warps][3][R] peer masks (kRankSmem)
 
+  dependents_may_start();
+  wait_for_previous_kernel();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   uint32_t n = a.n_ptr ? *a.n_ptr : a.capacity;
   if (n > a.capacity) n = a.capacity;
@@ -348,8 +353,7 @@ cudaError_t launch_pass_w(const PassArgs& p, uint32_t grid, cudaStream_t s) {
   const cudaError_t e = cudaFuncSetAttribute(k_onesweep<RB, PAY2, W>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k_onesweep<RB, PAY2, W><<<grid, kSortThreads, smem, s>>>(p);
-  return cudaGetLastError();
+  return launch_dependent(k_onesweep<RB, PAY2, W>, grid, kSortThreads, smem, s, p);
 }
 
 template <int RB, bool PAY2>

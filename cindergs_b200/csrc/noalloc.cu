@@ -103,6 +103,7 @@ extern "C" int cgs_sort_pairs_u32_noalloc(uint32_t* d_keys, uint32_t* d_vals, ui
   sa.radix_bits = rb;
   sa.hist = hist;
   sa.status = status;
+  sa.large_tiles = true;  // what kStatusBytes holds
   sa.tile_ctr = words + 2;
   sa.status_word = words + 1;
   sa.src = 0;

@@ -4,10 +4,10 @@
 // (render/kernels/radix_sort.rs:292-477), whose 4-bit passes each ran a
 // histogram kernel, a 1-3 level scan and a scatter kernel.
 //
-// Per pass and per 4096-key tile (256 threads x 16 keys, warp-striped so a
-// warp's item j is 32 consecutive keys):
+// Per pass and per tile of 2048 or 4096 keys (256 threads x 8 or 16 keys, warp-
+// striped so a warp's item j is 32 consecutive keys):
 //   1. keys and payloads are loaded coalesced into registers;
-//   2. each warp ranks its 512 keys by digit, 32 at a time (the lanes sharing
+//   2. each warp ranks its 256 or 512 keys by digit, 32 at a time (the lanes sharing
 //      a digit found by __match_any_sync, by one ballot per digit bit, or by
 //      shared-memory peer masks, chosen per pass), keeping a per-warp digit
 //      counter in shared memory (stable: ranks follow key order);
@@ -33,13 +33,21 @@ namespace cgs {
 namespace {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;  // 4096
 constexpr int kSortWarps = kSortThreads / 32;
 // Reorder buffers hold one padding word per 32 keys: the lanes of a warp
 // whose keys fall in different digits write positions about one digit run
 // (~32 keys) apart, which without padding map to the same bank.
-constexpr uint32_t kSortTileP = kSortTile + kSortTile / 32;
+constexpr uint32_t sort_tile_padded(int items) { return kSortThreads * items + kSortThreads * items / 32; }
+// Keys per thread. A tile of 16 keys a thread ranks them one after another and
+// leaves SMs idle below about 148 tiles; one of 8 has twice the blocks and half
+// that chain, but twice the look-back. Measured with 8 / 16 (4) keys a thread:
+// three 8-bit passes of 20k pairs 94 / 97 (93) us with the call around them,
+// of 300k 113 / 122 (121), 600k 121 / 121 (134), 1.2M 139 / 136 (160), 3M 196 /
+// 185 (235); a frame's splat sort, 20k 24 / 31 (24) us, 1.1M in a capacity of
+// 1.4M 55 / 63 (68) us. The line lies where the frame's sorts, whose narrower
+// digits look back less, still gain. It depends on the capacity alone, which
+// the look-back buffers are sized and cleared for.
+int sort_items(uint32_t capacity) { return capacity <= 3u << 19 ? 8 : 16; }
 __device__ __forceinline__ uint32_t padded(uint32_t i) { return i + (i >> 5); }
 // Look-back words: a flag (tile count published / inclusive prefix
 // published) above the count. 32-bit words carry counts below 2^30 (splat
@@ -91,6 +99,7 @@ struct PassArgs {
   uint32_t grid_tiles;     // tiles covered by the grid (all of clear_next)
   uint32_t* tile_ctr;
   uint32_t* status_word;
+  uint32_t items;          // keys per thread: 8 or 16
   uint32_t rank;           // how a warp finds the lanes sharing a digit: kRank*
   // last pass of a sort with ranges: per screen tile (key >> tile_shift,
   // below num_tiles), atomicMax of the complemented first entry and of the
@@ -144,9 +153,11 @@ __device__ __forceinline__ uint32_t digit_lookback(const W* status, uint32_t til
   return excl;
 }
 
-template <int RB, bool PAY2, typename W>
+template <int ITEMS, int RB, bool PAY2, typename W>
 __global__ void __launch_bounds__(kSortThreads, PAY2 ? 3 : 4) k_onesweep(const PassArgs a) {
   constexpr uint32_t R = 1u << RB;
+  constexpr int kSortItems = ITEMS;
+  constexpr uint32_t kSortTile = kSortThreads * ITEMS, kSortTileP = sort_tile_padded(ITEMS);
   W* const lb = static_cast<W*>(a.status);
   static_assert(R <= (uint32_t)kSortThreads, "one thread per digit");
   extern __shared__ __align__(16) uint32_t smem[];
@@ -168,7 +179,8 @@ __global__ void __launch_bounds__(kSortThreads, PAY2 ? 3 : 4) k_onesweep(const P
   if (tid == 0) s_misc[0] = atomicAdd(a.tile_ctr, 1u);
   for (uint32_t k = tid; k < kSortWarps * R; k += kSortThreads) s_whist[k] = 0u;
   if (a.rank == kRankSmem)
-    for (uint32_t k = tid; k < kSortWarps * 3 * R; k += kSortThreads) s_wor[k] = 0u;
+    for (uint32_t k = tid; k < kSortWarps * 3 * R / 4; k += kSortThreads)
+      reinterpret_cast<uint4*>(s_wor)[k] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
   const uint32_t tile = s_misc[0];
   // Clear this tile's words of the other look-back buffer for the next pass
@@ -339,27 +351,28 @@ __global__ void __launch_bounds__(kSortThreads, PAY2 ? 3 : 4) k_onesweep(const P
   if (bad) atomicOr(a.status_word, kStatusCapacity);
 }
 
-template <int RB, bool PAY2>
+template <int ITEMS, int RB, bool PAY2>
 size_t onesweep_smem(uint32_t rank) {
   constexpr uint32_t R = 1u << RB;
-  return sizeof(uint32_t) * ((PAY2 ? 3 : 2) * kSortTileP + kSortWarps * R + 3 * R + 48 +
+  return sizeof(uint32_t) * ((PAY2 ? 3 : 2) * sort_tile_padded(ITEMS) + kSortWarps * R + 3 * R + 48 +
                              (rank == kRankSmem ? kSortWarps * 3 * R : 0u));
 }
 
-template <int RB, bool PAY2, typename W>
+template <int ITEMS, int RB, bool PAY2, typename W>
 cudaError_t launch_pass_w(const PassArgs& p, uint32_t grid, cudaStream_t s) {
-  const size_t smem = onesweep_smem<RB, PAY2>(p.rank);
+  const size_t smem = onesweep_smem<ITEMS, RB, PAY2>(p.rank);
   // per device: set on every launch (a host-side attribute write)
-  const cudaError_t e = cudaFuncSetAttribute(k_onesweep<RB, PAY2, W>,
+  const cudaError_t e = cudaFuncSetAttribute(k_onesweep<ITEMS, RB, PAY2, W>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  return launch_dependent(k_onesweep<RB, PAY2, W>, grid, kSortThreads, smem, s, p);
+  return launch_dependent(k_onesweep<ITEMS, RB, PAY2, W>, grid, kSortThreads, smem, s, p);
 }
 
 template <int RB, bool PAY2>
 cudaError_t launch_pass(const PassArgs& p, uint32_t grid, bool wide, cudaStream_t s) {
-  return wide ? launch_pass_w<RB, PAY2, unsigned long long>(p, grid, s)
-              : launch_pass_w<RB, PAY2, uint32_t>(p, grid, s);
+  if (p.items == 8) return launch_pass_w<8, RB, PAY2, uint32_t>(p, grid, s);
+  return wide ? launch_pass_w<16, RB, PAY2, unsigned long long>(p, grid, s)
+              : launch_pass_w<16, RB, PAY2, uint32_t>(p, grid, s);
 }
 
 // Digit histograms of every pass in one read of the keys.
@@ -404,7 +417,10 @@ cudaError_t launch_drill_digit_lookback(const uint32_t* status, uint32_t radix,
   return cudaGetLastError();
 }
 
-uint32_t sort_tiles(uint32_t capacity) { return (capacity + kSortTile - 1) / kSortTile; }
+uint32_t sort_tiles(uint32_t capacity) {
+  const uint32_t tile = kSortThreads * sort_items(capacity);
+  return (capacity + tile - 1) / tile;
+}
 
 uint32_t sort_passes(uint32_t num_bits, uint32_t radix_bits) {
   return (num_bits + radix_bits - 1) / radix_bits;
@@ -422,11 +438,13 @@ cudaError_t run_radix_sort(const SortArgs& a, int* out_src, cudaStream_t s) {
   const uint32_t rb = a.radix_bits < 4 ? 4u : (a.radix_bits > 8 ? 8u : a.radix_bits);
   const uint32_t R = 1u << rb;
   const uint32_t passes = sort_passes(a.num_bits, rb);
-  const uint32_t tiles = sort_tiles(a.capacity);
+  const int items = a.large_tiles ? 16 : sort_items(a.capacity);
+  const uint32_t keys = kSortThreads * items, tiles = (a.capacity + keys - 1) / keys;
   int src = a.src;
   const bool pay2 = a.vals2[0] != nullptr;
   const bool wide = a.wide_lookback;
   if (!wide && a.capacity > (1u << 30)) return cudaErrorInvalidValue;  // 30-bit counts
+  if (wide && items != 16) return cudaErrorInvalidValue;  // no such kernel
   for (uint32_t p = 0; p < passes; ++p) {
     PassArgs pa;
     pa.keys_in = a.keys[src];
@@ -454,6 +472,7 @@ cudaError_t run_radix_sort(const SortArgs& a, int* out_src, cudaStream_t s) {
     }
     if (pa.clear_stride < R && pa.clear_next) return cudaErrorInvalidValue;
     pa.grid_tiles = tiles;
+    pa.items = (uint32_t)items;
     pa.tile_ctr = a.tile_ctr + p;
     pa.status_word = a.status_word;
     pa.rank = ((a.smem_mask >> p) & 1u) ? kRankSmem : (((a.ballot_mask >> p) & 1u) ? kRankBallot : kRankMatch);

@@ -15,8 +15,9 @@ namespace cgs {
 // one shared-memory size, where it hides about 1.2 us of each launch: the
 // training step (13 launches, 184 -> 167 us) and the sort's passes. Between
 // the frame's other kernels it costs more than it gives in large frames (12
-// views of 2M splats 6.8 -> 8.6 ms, 1.1M splats 556 -> 605 us): blocks that
-// wait take shared memory from the L1 cache of the kernel still running.
+// views of 2M splats 6.8 -> 8.6 ms, 1.1M splats 556 -> 605 us), probably
+// because blocks that wait take shared memory from the L1 cache of the kernel
+// still running.
 template <typename... P, typename... A>
 cudaError_t launch_dependent(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};

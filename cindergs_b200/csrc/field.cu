@@ -15,7 +15,7 @@ namespace cgs {
     if (e_ != cudaSuccess) return e_;  \
   } while (0)
 
-cudaError_t FieldBuf::ensure(size_t bytes) {
+cudaError_t FieldBuf::ensure(size_t bytes, cudaStream_t s) {
   if (bytes == 0) bytes = 16;
   if (bytes <= cap) return cudaSuccess;
   if (p) cudaFree(p);
@@ -23,7 +23,7 @@ cudaError_t FieldBuf::ensure(size_t bytes) {
   cap = 0;
   FIELD_TRY(cudaMalloc(&p, bytes));
   cap = bytes;
-  return cudaMemset(p, 0, bytes);
+  return cudaMemsetAsync(p, 0, bytes, s);
 }
 
 namespace {
@@ -115,19 +115,19 @@ cudaError_t FieldState::init(uint32_t nv, const float* rest_v4, uint64_t seed, c
   }
   for (uint32_t i = 0; i < sizes[kW5]; ++i) h[off[kW5] + i] = (float)(1e-3 * normal(st));
   for (uint32_t j = 0; j < nv; ++j) h[off[kB5] + j] = 1.0f / (float)nv;
-  FIELD_TRY(p32.ensure((size_t)o * 4));
-  FIELD_TRY(g32.ensure((size_t)o * 4));
-  FIELD_TRY(m1.ensure((size_t)o * 4));
-  FIELD_TRY(m2.ensure((size_t)o * 4));
-  FIELD_TRY(pb.ensure((size_t)o * 2));
-  FIELD_TRY(enc_d.ensure(16));
-  FIELD_TRY(M_d.ensure(64));
-  FIELD_TRY(rest_d.ensure((size_t)nv * 16));
-  FIELD_TRY(proj.ensure((size_t)kFieldProj * 4));
-  FIELD_TRY(proj_rest.ensure((size_t)kFieldProj * 4));
-  FIELD_TRY(loss.ensure(16));
-  FIELD_TRY(status.ensure(16));
-  FIELD_TRY(wT.ensure((size_t)kFieldHid * (3 * kFieldHid + ldV) * 2));
+  FIELD_TRY(p32.ensure((size_t)o * 4, s));
+  FIELD_TRY(g32.ensure((size_t)o * 4, s));
+  FIELD_TRY(m1.ensure((size_t)o * 4, s));
+  FIELD_TRY(m2.ensure((size_t)o * 4, s));
+  FIELD_TRY(pb.ensure((size_t)o * 2, s));
+  FIELD_TRY(enc_d.ensure(16, s));
+  FIELD_TRY(M_d.ensure(64, s));
+  FIELD_TRY(rest_d.ensure((size_t)nv * 16, s));
+  FIELD_TRY(proj.ensure((size_t)kFieldProj * 4, s));
+  FIELD_TRY(proj_rest.ensure((size_t)kFieldProj * 4, s));
+  FIELD_TRY(loss.ensure(16, s));
+  FIELD_TRY(status.ensure(16, s));
+  FIELD_TRY(wT.ensure((size_t)kFieldHid * (3 * kFieldHid + ldV) * 2, s));
   FIELD_TRY(cudaMemsetAsync(m1.p, 0, (size_t)o * 4, s));
   FIELD_TRY(cudaMemsetAsync(m2.p, 0, (size_t)o * 4, s));
   FIELD_TRY(cudaMemsetAsync(g32.p, 0, (size_t)o * 4, s));
@@ -157,29 +157,29 @@ FieldNet FieldState::net() const {
   return n;
 }
 
-cudaError_t FieldState::ensure_batch(uint32_t B, bool train) {
+cudaError_t FieldState::ensure_batch(uint32_t B, bool train, cudaStream_t s) {
   const size_t b = B, H = kFieldHid;
   if (B > Bcap) {
-    FIELD_TRY(x.ensure(b * 12));
-    FIELD_TRY(idx.ensure(b * 4));
-    FIELD_TRY(a0.ensure(b * kFieldIn * 2));
+    FIELD_TRY(x.ensure(b * 12, s));
+    FIELD_TRY(idx.ensure(b * 4, s));
+    FIELD_TRY(a0.ensure(b * kFieldIn * 2, s));
     for (int l = 0; l < 4; ++l) {
-      FIELD_TRY(pre[l].ensure(b * H * 4));
-      FIELD_TRY(h[l].ensure(b * H * 2));
+      FIELD_TRY(pre[l].ensure(b * H * 4, s));
+      FIELD_TRY(h[l].ensure(b * H * 2, s));
     }
-    FIELD_TRY(z.ensure(b * ldV * 4));
+    FIELD_TRY(z.ensure(b * ldV * 4, s));
     Bcap = B;
   }
   if (train && B > Btrain) {
-    FIELD_TRY(dzb.ensure(b * ldV * 2));
-    for (int l = 0; l < 2; ++l) FIELD_TRY(dpreb[l].ensure(b * H * 2));
+    FIELD_TRY(dzb.ensure(b * ldV * 2, s));
+    for (int l = 0; l < 2; ++l) FIELD_TRY(dpreb[l].ensure(b * H * 2, s));
     for (int l = 0; l < 5; ++l) {
-      FIELD_TRY(inT[l].ensure((l == 0 ? kFieldIn : H) * b * 2));
-      FIELD_TRY(dT[l].ensure((l == 4 ? ldV : H) * b * 2));
-      if (l < 4) FIELD_TRY(dpre[l].ensure(b * H * 4));
+      FIELD_TRY(inT[l].ensure((l == 0 ? kFieldIn : H) * b * 2, s));
+      FIELD_TRY(dT[l].ensure((l == 4 ? ldV : H) * b * 2, s));
+      if (l < 4) FIELD_TRY(dpre[l].ensure(b * H * 4, s));
     }
-    FIELD_TRY(dz.ensure(b * ldV * 4));
-    FIELD_TRY(gemm_ws.ensure((size_t)16 * (H * kFieldIn + 3 * H * H + (size_t)V * H) * 4));
+    FIELD_TRY(dz.ensure(b * ldV * 4, s));
+    FIELD_TRY(gemm_ws.ensure((size_t)16 * (H * kFieldIn + 3 * H * H + (size_t)V * H) * 4, s));
     Btrain = B;
   }
   return cudaSuccess;
@@ -199,7 +199,7 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
                                 uint32_t seed, const float4* rest_verts, float lambda,
                                 cudaStream_t s) {
   const bool train = target != nullptr;
-  FIELD_TRY(ensure_batch(B, train));
+  FIELD_TRY(ensure_batch(B, train, s));
   FieldBatch fb{};
   fb.points = points;
   fb.n = n;

@@ -17,7 +17,10 @@ struct FieldBuf {
   ~FieldBuf() {
     if (p) cudaFree(p);
   }
-  cudaError_t ensure(size_t bytes);  // grows, zero-filled; contents are not kept
+  // grows; zero-filled on stream s (a clear on the legacy stream would not be
+  // ordered with the kernels of a context's own, non-blocking stream);
+  // contents are not kept
+  cudaError_t ensure(size_t bytes, cudaStream_t s);
   template <typename T>
   T* as() const {
     return reinterpret_cast<T*>(p);
@@ -50,7 +53,7 @@ struct FieldState {
   // output weights N(0, 1e-6), output biases 1/V (uniform weights).
   cudaError_t init(uint32_t V, const float* rest_v4, uint64_t seed, cudaStream_t s);
   FieldNet net() const;
-  cudaError_t ensure_batch(uint32_t B, bool train);
+  cudaError_t ensure_batch(uint32_t B, bool train, cudaStream_t s);
   // Forward over a batch (rows r -> points as FieldBatch::seed says), with
   // the loss and dL/dz when target is given. loss[0..1] accumulate in `loss`.
   cudaError_t forward(const float* points, const float* target, uint32_t n, uint32_t B,

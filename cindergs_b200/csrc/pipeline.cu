@@ -1085,7 +1085,7 @@ int cgs_ctx_create(int device, void* stream, cgs_ctx** out_ctx) {
   }
   // persistent words: [0] split count
   if (ctx->ensure(ctx->persist, 256, "persistent words") != CGS_OK ||
-      cudaMemset(ctx->persist.p, 0, 256) != cudaSuccess) {
+      cudaMemsetAsync(ctx->persist.p, 0, 256, ctx->stream) != cudaSuccess) {
     delete ctx;
     return CGS_E_OOM;
   }

@@ -157,32 +157,35 @@ FieldNet FieldState::net() const {
   return n;
 }
 
-cudaError_t FieldState::ensure_batch(uint32_t B, bool train, cudaStream_t s) {
+BatchLayout::BatchLayout(uint32_t B, uint32_t V, uint32_t ldV, bool train) {
+  size_t at = 0;
+  auto take = [&](size_t n) {
+    const size_t p = at;
+    at = (at + n + 255) & ~(size_t)255;
+    return p;
+  };
   const size_t b = B, H = kFieldHid;
-  if (B > Bcap) {
-    FIELD_TRY(x.ensure(b * 12, s));
-    FIELD_TRY(idx.ensure(b * 4, s));
-    FIELD_TRY(a0.ensure(b * kFieldIn * 2, s));
-    for (int l = 0; l < 4; ++l) {
-      FIELD_TRY(pre[l].ensure(b * H * 4, s));
-      FIELD_TRY(h[l].ensure(b * H * 2, s));
-    }
-    FIELD_TRY(z.ensure(b * ldV * 4, s));
-    Bcap = B;
+  x = take(b * 12);
+  idx = take(b * 4);
+  a0 = take(b * kFieldIn * 2);
+  for (int l = 0; l < 4; ++l) {
+    pre[l] = take(b * H * 4);
+    h[l] = take(b * H * 2);
   }
-  if (train && B > Btrain) {
-    FIELD_TRY(dzb.ensure(b * ldV * 2, s));
-    for (int l = 0; l < 2; ++l) FIELD_TRY(dpreb[l].ensure(b * H * 2, s));
+  z = take(b * ldV * 4);
+  if (train) {
+    dzb = take(b * ldV * 2);
+    for (int l = 0; l < 2; ++l) dpreb[l] = take(b * H * 2);
     for (int l = 0; l < 5; ++l) {
-      FIELD_TRY(inT[l].ensure((l == 0 ? kFieldIn : H) * b * 2, s));
-      FIELD_TRY(dT[l].ensure((l == 4 ? ldV : H) * b * 2, s));
-      if (l < 4) FIELD_TRY(dpre[l].ensure(b * H * 4, s));
+      inT[l] = take((l == 0 ? kFieldIn : H) * b * 2);
+      dT[l] = take((l == 4 ? ldV : H) * b * 2);
+      if (l < 4) dpre[l] = take(b * H * 4);
     }
-    FIELD_TRY(dz.ensure(b * ldV * 4, s));
-    FIELD_TRY(gemm_ws.ensure((size_t)16 * (H * kFieldIn + 3 * H * H + (size_t)V * H) * 4, s));
-    Btrain = B;
+    dz = take(b * ldV * 4);
+    for (int l = 0; l < 5; ++l)
+      ws[l] = take((size_t)grad_splits(B) * (l == 4 ? V : H) * (l == 0 ? kFieldIn : H) * 4);
   }
-  return cudaSuccess;
+  bytes = at;
 }
 
 void FieldState::transposed(__nv_bfloat16* (&w)[4]) const {
@@ -199,17 +202,18 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
                                 uint32_t seed, const float4* rest_verts, float lambda,
                                 cudaStream_t s) {
   const bool train = target != nullptr;
-  FIELD_TRY(ensure_batch(B, train, s));
+  const BatchLayout L(B, V, ldV, train);
+  FIELD_TRY(batch.ensure(L.bytes, s));
   FieldBatch fb{};
   fb.points = points;
   fb.n = n;
   fb.B = B;
   fb.seed = seed;
   fb.enc = enc_d.as<float>();
-  fb.x = x.as<float>();
-  fb.idx = idx.as<uint32_t>();
-  fb.a0 = a0.as<__nv_bfloat16>();
-  fb.a0T = train ? inT[0].as<__nv_bfloat16>() : nullptr;
+  fb.x = batch.at<float>(L.x);
+  fb.idx = batch.at<uint32_t>(L.idx);
+  fb.a0 = batch.at<__nv_bfloat16>(L.a0);
+  fb.a0T = train ? batch.at<__nv_bfloat16>(L.inT[0]) : nullptr;
   FIELD_TRY(launch_field_gather(fb, s));
   const FieldNet nt = net();
   const __nv_bfloat16* W[4] = {nt.W1b, nt.W2b, nt.W3b, nt.W4b};
@@ -217,39 +221,39 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
   for (int l = 0; l < 4; ++l) {
     GemmArgs g{};
     g.status = status.as<uint32_t>();
-    g.A = l == 0 ? a0.as<__nv_bfloat16>() : h[l - 1].as<__nv_bfloat16>();
+    g.A = batch.at<__nv_bfloat16>(l == 0 ? L.a0 : L.h[l - 1]);
     g.lda = g.K = l == 0 ? kFieldIn : kFieldHid;
     g.B = W[l];
     g.ldb = g.K;
     g.M = B;
     g.N = kFieldHid;
-    g.C = pre[l].as<float>();
+    g.C = batch.at<float>(L.pre[l]);
     g.ldc = kFieldHid;
     g.bias = bias[l];
-    g.D = h[l].as<__nv_bfloat16>();
+    g.D = batch.at<__nv_bfloat16>(L.h[l]);
     g.ldd = kFieldHid;
-    g.DT = train ? inT[l + 1].as<__nv_bfloat16>() : nullptr;
+    g.DT = train ? batch.at<__nv_bfloat16>(L.inT[l + 1]) : nullptr;
     g.ldt = B;
     FIELD_TRY(launch_gemm_nt(g, kEpiBiasSilu, s));
   }
   GemmArgs g{};
   g.status = status.as<uint32_t>();
-  g.A = h[3].as<__nv_bfloat16>();
+  g.A = batch.at<__nv_bfloat16>(L.h[3]);
   g.lda = g.K = kFieldHid;
   g.B = nt.W5b;
   g.ldb = kFieldHid;
   g.M = B;
   g.N = V;
-  g.C = z.as<float>();
+  g.C = batch.at<float>(L.z);
   g.ldc = ldV;
   g.bias = nt.b5;
   FIELD_TRY(launch_gemm_nt(g, kEpiBias, s));
   if (!target) return cudaSuccess;
   FieldLoss fl{};
-  fl.z = z.as<float>();
+  fl.z = batch.at<float>(L.z);
   fl.target = target;
-  fl.idx = idx.as<uint32_t>();
-  fl.x = x.as<float>();
+  fl.idx = batch.at<uint32_t>(L.idx);
+  fl.x = batch.at<float>(L.x);
   fl.verts = rest_verts;
   fl.B = B;
   fl.V = V;
@@ -257,53 +261,52 @@ cudaError_t FieldState::forward(const float* points, const float* target, uint32
   fl.lambda = lambda;
   fl.s2 = scale * scale;
   std::memcpy(fl.M, M.m, 64);
-  fl.dzb = dzb.as<__nv_bfloat16>();
-  fl.dzT = dT[4].as<__nv_bfloat16>();
-  fl.dz = dz.as<float>();
+  fl.dzb = batch.at<__nv_bfloat16>(L.dzb);
+  fl.dzT = batch.at<__nv_bfloat16>(L.dT[4]);
+  fl.dz = batch.at<float>(L.dz);
   fl.loss = loss.as<float>();
   return launch_field_loss(fl, s);
 }
 
 cudaError_t FieldState::backward(uint32_t B, cudaStream_t s) {
   if (B % 8) return cudaErrorInvalidValue;  // transposed operands have row length B
+  const BatchLayout L(B, V, ldV, true);
   __nv_bfloat16* w[4];
   transposed(w);
   // dL/dpre of layer l = (dL/dz or dL/dpre of the layer above) W silu'(pre_l)
   for (int l = 3; l >= 0; --l) {
     GemmArgs g{};
     g.status = status.as<uint32_t>();
-    g.A = l == 3 ? dzb.as<__nv_bfloat16>() : dpreb[(l + 1) & 1].as<__nv_bfloat16>();
+    g.A = batch.at<__nv_bfloat16>(l == 3 ? L.dzb : L.dpreb[(l + 1) & 1]);
     g.lda = l == 3 ? ldV : kFieldHid;
     g.K = l == 3 ? V : kFieldHid;
     g.B = w[l];
     g.ldb = g.lda;
     g.M = B;
     g.N = kFieldHid;
-    g.pre = pre[l].as<float>();
-    g.C = dpre[l].as<float>();
+    g.pre = batch.at<float>(L.pre[l]);
+    g.C = batch.at<float>(L.dpre[l]);
     g.ldc = kFieldHid;
-    g.D = l > 0 ? dpreb[l & 1].as<__nv_bfloat16>() : nullptr;
+    g.D = l > 0 ? batch.at<__nv_bfloat16>(L.dpreb[l & 1]) : nullptr;
     g.ldd = kFieldHid;
-    g.DT = dT[l].as<__nv_bfloat16>();
+    g.DT = batch.at<__nv_bfloat16>(L.dT[l]);
     g.ldt = B;
     FIELD_TRY(launch_gemm_nt(g, kEpiBack, s));
   }
   // dW_l = (dL/dpre_l or dL/dz)^T (input of the layer), db_l = their column sums
   GemmBatch gb{};
   gb.splits = grad_splits(B);
-  float* ws = gemm_ws.as<float>();
   for (int l = 0; l < 5; ++l) {
     GemmArgs& g = gb.g[l];
     g.status = status.as<uint32_t>();
-    g.A = dT[l].as<__nv_bfloat16>();
-    g.B = inT[l].as<__nv_bfloat16>();
+    g.A = batch.at<__nv_bfloat16>(L.dT[l]);
+    g.B = batch.at<__nv_bfloat16>(L.inT[l]);
     g.lda = g.ldb = g.K = B;
     g.M = l == 4 ? V : kFieldHid;
     g.N = l == 0 ? kFieldIn : kFieldHid;
-    g.C = ws;
-    ws += (size_t)16 * g.M * g.N;
+    g.C = batch.at<float>(L.ws[l]);
     gb.first[l + 1] = gb.first[l] + (g.M + 127) / 128 * ((g.N + 63) / 64);
-    gb.sum[l] = l == 4 ? dz.as<float>() : dpre[l].as<float>();
+    gb.sum[l] = batch.at<float>(l == 4 ? L.dz : L.dpre[l]);
     gb.sum_n[l] = g.M;
     gb.sum_ld[l] = l == 4 ? ldV : kFieldHid;
     gb.sum_out[l] = g32.as<float>() + off[2 * l + 1];
@@ -317,11 +320,8 @@ cudaError_t FieldState::update(uint32_t B, float lr, cudaStream_t s) {
   u.V = V;
   u.ldV = ldV;
   u.splits = grad_splits(B);
-  const float* ws = gemm_ws.as<float>();
-  for (int l = 0; l < 5; ++l) {
-    u.ws[l] = ws;
-    ws += (size_t)16 * (l == 4 ? V : kFieldHid) * (l == 0 ? kFieldIn : kFieldHid);
-  }
+  const BatchLayout L(B, V, ldV, true);
+  for (int l = 0; l < 5; ++l) u.ws[l] = batch.at<float>(L.ws[l]);
   u.p = p32.as<float>();
   u.g = g32.as<float>();
   u.m = m1.as<float>();
@@ -346,7 +346,8 @@ cudaError_t FieldState::eval(uint32_t n, const float* points, float* w, cudaStre
   for (uint32_t done = 0; done < n; done += chunk) {
     const uint32_t B = std::min(chunk, n - done);
     FIELD_TRY(forward(points + 3 * (size_t)done, nullptr, B, B, 0, nullptr, 0.0f, s));
-    FIELD_TRY(launch_field_weights(z.as<float>(), B, V, ldV, x.as<float>(), rest_d.as<float4>(), M,
+    const BatchLayout L(B, V, ldV, false);
+    FIELD_TRY(launch_field_weights(batch.at<float>(L.z), B, V, ldV, batch.at<float>(L.x), rest_d.as<float4>(), M,
                                    w + (size_t)done * V, s));
   }
   return cudaSuccess;

@@ -25,6 +25,22 @@ struct FieldBuf {
   T* as() const {
     return reinterpret_cast<T*>(p);
   }
+  template <typename T>
+  T* at(size_t offset) const {
+    return reinterpret_cast<T*>(static_cast<char*>(p) + offset);
+  }
+};
+
+// Byte offsets of a batch's buffers in their one allocation (B rows; the
+// buffers from dzb on in training only). Worked out from the rows and the cage
+// at every use: a context's next cage may have more vertices at the same B.
+// inT: the transposed inputs of layers 1..5 (features, then h); dT: the
+// transposed dL/dpre of layers 1..4 and dL/dz; dpre, dz: the same in fp32; ws:
+// the weight gradients' partial sums over grad_splits(B) ranges of the batch.
+// A step writes every element that it reads.
+struct BatchLayout {
+  size_t x, idx, a0, pre[4], h[4], z, dzb, dpreb[2], inT[5], dT[5], dpre[4], dz, ws[5], bytes;
+  BatchLayout(uint32_t B, uint32_t V, uint32_t ldV, bool train);
 };
 
 // Parameter block (fp32 master copy, gradients, Adam moments and a bf16 copy
@@ -40,12 +56,7 @@ struct FieldState {
   FieldMat M{};             // (Vb Vb^T)^-1, Vb = [1; rest vertices]
   uint32_t step = 0;        // Adam steps taken
   FieldBuf p32, g32, m1, m2, pb, enc_d, M_d, rest_d, proj, proj_rest, loss, wT, status;  // wT: W2..W5 transposed
-  // training batch (B rows)
-  uint32_t Bcap = 0, Btrain = 0;
-  // inT: the transposed inputs of layers 1..5 (features, then h); dT: the
-  // transposed dL/dpre of layers 1..4 and dL/dz; dpre, dz: the same in fp32
-  FieldBuf x, idx, a0, pre[4], h[4], z, dz, dzb, dpre[4], dpreb[2], inT[5], dT[5];
-  FieldBuf gemm_ws;  // split-K partial sums of the weight gradients (K = batch)
+  FieldBuf batch;  // BatchLayout
 
   uint32_t total() const { return off[kFieldParams]; }
   // New network for a cage of V vertices with the given rest vertices [V*4]
@@ -53,7 +64,6 @@ struct FieldState {
   // output weights N(0, 1e-6), output biases 1/V (uniform weights).
   cudaError_t init(uint32_t V, const float* rest_v4, uint64_t seed, cudaStream_t s);
   FieldNet net() const;
-  cudaError_t ensure_batch(uint32_t B, bool train, cudaStream_t s);
   // Forward over a batch (rows r -> points as FieldBatch::seed says), with
   // the loss and dL/dz when target is given. loss[0..1] accumulate in `loss`.
   cudaError_t forward(const float* points, const float* target, uint32_t n, uint32_t B,

@@ -102,6 +102,7 @@ cudaError_t launch_mvc_residual(uint32_t nb, const uint32_t* list, const float4*
                                 uint32_t* flag, cudaStream_t s);
 
 // ---- learned MVC field (mvc_field.cu) ------------------------------------------
+constexpr uint32_t kMvcMaxVerts = 1024;  // vertices of a polygon cage (mvc_cage_fits)
 constexpr int kFieldBands = 8;
 constexpr int kFieldIn = 64;    // 3 + 6 * bands, zero-padded
 constexpr int kFieldHid = 128;

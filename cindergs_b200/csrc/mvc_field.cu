@@ -735,14 +735,14 @@ cudaError_t launch_field_refresh(const uint32_t* off, uint32_t V, uint32_t ldV, 
 
 cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s) {
   if (l.B == 0) return cudaSuccess;
-  if (l.V > 1024u || (l.B & 1u)) return cudaErrorInvalidValue;
+  if (l.V > kMvcMaxVerts || (l.B & 1u)) return cudaErrorInvalidValue;
   const size_t smem = (size_t)l.V * (16 + 2 * kLossRows);
   auto run = [&](auto kernel) {
-    if (smem > 48 * 1024) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+    // 48 KB at 1,024 vertices, beside the block's static words: past what a
+    // launch may have without the opt-in from 1,022 vertices on
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)(kMvcMaxVerts * (16 + 2 * kLossRows)));
+    if (e != cudaSuccess) return e;
     return launch_dependent(kernel, (l.B + kLossRows - 1) / kLossRows, 32 * kLossRows, smem, s, l);
   };
   if (l.V <= 192u) return run(k_field_loss<6>);

@@ -161,6 +161,7 @@ __device__ __forceinline__ void mvc_eval(const MvcCage& c, F3 x, const EvalSmem&
 }
 
 constexpr int kMaxOwn = 8;  // V <= 8 * 128
+static_assert(kMaxOwn * kMvcThreads == (int)kMvcMaxVerts, "a thread's vertices");
 
 __device__ __forceinline__ EvalSmem eval_smem(unsigned char* base, const MvcCage& c) {
   EvalSmem s;
@@ -357,7 +358,7 @@ cudaError_t set_smem(K kernel, size_t bytes) {
 }  // namespace
 
 bool mvc_cage_fits(uint32_t V, uint32_t F) {
-  return V >= 4 && F >= 4 && V <= (uint32_t)kMaxOwn * kMvcThreads && (V + F) * 16 + 32 <= 200 * 1024;
+  return V >= 4 && F >= 4 && V <= kMvcMaxVerts && (V + F) * 16 + 32 <= 200 * 1024;
 }
 
 cudaError_t launch_mvc_weights(const MvcCage& c, uint32_t n, const float* pts, float* w,

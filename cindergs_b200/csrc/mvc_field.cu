@@ -757,9 +757,12 @@ cudaError_t launch_field_update(const FieldUpdate& u, cudaStream_t s) {
 cudaError_t launch_field_project(const FieldNet& net, uint32_t V, const float4* rest,
                                  const float4* verts, const float* M, float* proj,
                                  cudaStream_t s) {
+  // the opt-in is the same for every cage: another thread's launch may come
+  // between it and this one
+  if (V > kMvcMaxVerts) return cudaErrorInvalidValue;
   const size_t smem = (size_t)V * 48;
   const cudaError_t e = cudaFuncSetAttribute(
-      k_field_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      k_field_project, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMvcMaxVerts * 48));
   if (e != cudaSuccess) return e;
   k_field_project<<<kHid / kProjUnits, kProjThreads, smem, s>>>(net, V, rest, verts, M, proj);
   return cudaGetLastError();

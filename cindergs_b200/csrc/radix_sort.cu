@@ -361,9 +361,11 @@ size_t onesweep_smem(uint32_t rank) {
 template <int ITEMS, int RB, bool PAY2, typename W>
 cudaError_t launch_pass_w(const PassArgs& p, uint32_t grid, cudaStream_t s) {
   const size_t smem = onesweep_smem<ITEMS, RB, PAY2>(p.rank);
-  // per device: set on every launch (a host-side attribute write)
+  // per device: set on every launch (a host-side attribute write), to the same
+  // value, since another thread's launch may come between it and this one
   const cudaError_t e = cudaFuncSetAttribute(k_onesweep<ITEMS, RB, PAY2, W>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)onesweep_smem<ITEMS, RB, PAY2>(kRankSmem));
   if (e != cudaSuccess) return e;
   return launch_dependent(k_onesweep<ITEMS, RB, PAY2, W>, grid, kSortThreads, smem, s, p);
 }

@@ -349,16 +349,19 @@ __global__ void __launch_bounds__(kJacThreads) k_mvc_jacobian(uint32_t V, const 
 
 size_t eval_smem_bytes(const MvcCage& c) { return (size_t)(c.V + c.F) * 16 + 32; }
 
+// Opt-in for launches of any cage that mvc_cage_fits admits: the same value
+// every time, since another thread's launch may come between it and this one.
+constexpr uint32_t kMvcMaxSmem = 200 * 1024;
 template <typename K>
 cudaError_t set_smem(K kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (bytes > kMvcMaxSmem) return cudaErrorInvalidValue;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMvcMaxSmem);
 }
 
 }  // namespace
 
 bool mvc_cage_fits(uint32_t V, uint32_t F) {
-  return V >= 4 && F >= 4 && V <= kMvcMaxVerts && (V + F) * 16 + 32 <= 200 * 1024;
+  return V >= 4 && F >= 4 && V <= kMvcMaxVerts && (V + F) * 16 + 32 <= kMvcMaxSmem;
 }
 
 cudaError_t launch_mvc_weights(const MvcCage& c, uint32_t n, const float* pts, float* w,

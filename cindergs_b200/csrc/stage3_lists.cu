@@ -473,11 +473,10 @@ cudaError_t launch_list_pairs(const ListArgs& a, cudaStream_t s) {
   if (a.num_blocks == 0 || a.num_blocks > kListMaxBlocks) return cudaErrorInvalidValue;
   const size_t fixed = 4 * (3 * (size_t)kListSlots + 64);
   const size_t smem = sizeof(uint32_t) * std::max<uint32_t>(a.num_blocks, a.passes << a.radix_bits);
-  if (fixed + smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_list_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  // the same value for every viewport: another thread's launch may come between
+  const cudaError_t e = cudaFuncSetAttribute(k_list_pairs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)(sizeof(uint32_t) * kListMaxBlocks));
+  if (e != cudaSuccess) return e;
   // eight blocks of 256 threads per SM, fewer where the block counters are large
   const uint32_t per_sm = (uint32_t)std::min<size_t>(8, 227 * 1024 / (fixed + smem + 1024));
   const uint32_t tiles = (a.max_n + kListSlots - 1) / kListSlots;

@@ -281,19 +281,22 @@ struct cgs_ctx {
   bool last_f32 = false, frame_done = false;
   int latest_slot = -1;
   uint64_t frame_seq = 0;        // frames enqueued by cgs_execute_frame
-  uint64_t rerun_count = 0;      // Stage 3/4 re-runs after an entry overflow
-  uint64_t rerun_seq = 0;        // frame number of the latest re-run
   // Asynchronous RGBA8 readbacks (cgs_readback_rgba8_async): a device
   // snapshot of the framebuffer per slot, copied to the host on rb_stream.
   struct Readback {
     DevBuf stage;
     cudaEvent_t ready = nullptr, done = nullptr;
-    uint64_t ticket = 0, frame_seq = 0, reruns = 0;
+    uint64_t ticket = 0, frame_seq = 0;
     uint8_t* dst = nullptr;
     uint32_t W = 0, H = 0;
     int frame_slot = -1;
     bool pending = false;
+    bool stale = false;  // the snapshot holds a frame whose entries overflowed
   } rb[2];
+  void snapshots_stale(uint64_t seq) {  // of frame seq: it has to be copied again
+    for (auto& r : rb)
+      if (r.frame_seq == seq) r.stale = true;
+  }
   cudaStream_t rb_stream = nullptr;
   uint64_t rb_tickets = 0;
   // in-flight frames
@@ -309,15 +312,14 @@ struct cgs_ctx {
     cudaEvent_t kev[2 * kMaxMarks] = {};
     int kid[kMaxMarks] = {};
     int kcount = 0;
-    // what it takes to render the frame again after its tile entries
-    // overflowed while later frames were in flight: its arguments and the
-    // cage vertices it deformed with (device snapshots)
+    // what it takes to render the frame again for a readback, after its tile
+    // entries overflowed: its arguments and the cage vertices it deformed with
+    // (device snapshots)
     cgs_camera cam{};
     cgs_compositor comp{};
     cgs_frame_params params{};
     DevBuf verts_snap, mvc_snap;
     size_t verts_bytes = 0, mvc_bytes = 0;
-    bool overflowed = false;
   } ring[kRing];
   // The arena holds an earlier frame's intermediates (a re-render), not the
   // last frame's, until the next frame.
@@ -886,8 +888,7 @@ int rerun_stage34(cgs_ctx* ctx) {
                              cudaMemcpyDeviceToHost, ctx->stream), "read counters");
     CGS_CUDA(cudaStreamSynchronize(ctx->stream), "stage 3 re-run");
     ctx->s3_src = src;
-    ++ctx->rerun_count;
-    ctx->rerun_seq = ctx->ring[ctx->latest_slot].seq;
+    ctx->snapshots_stale(ctx->ring[ctx->latest_slot].seq);
     if (!(f.status & kStatusCapacity)) return CGS_OK;
   }
   return ctx->fail(CGS_E_CAPACITY, "tile entries still exceed the grown buffers");
@@ -921,7 +922,7 @@ int check_slot(cgs_ctx* ctx, int k, bool block) {
     } else {
       // a later frame is in flight: its pixels are rendered again if a
       // readback waits for them (rerender_slot); the buffers grow now
-      p.overflowed = true;
+      ctx->snapshots_stale(p.seq);
       grow_caps(ctx, h.fc, 100, 30);
     }
   } else if (p.stage3_ran) {
@@ -2385,6 +2386,9 @@ int cgs_execute_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_composit
   const int slot = ctx->next_slot;
   CGS_TRY(check_slot(ctx, slot, true));
   CGS_TRY(drain(ctx, false));
+  // a copy of that frame that has to be made again needs the slot's arguments
+  for (auto& r : ctx->rb)
+    if (r.pending && r.stale && r.frame_slot == slot) CGS_TRY(cgs_readback_wait(ctx, r.ticket));
   ctx->next_slot = (slot + 1) % kRing;
 
   cgs_ctx::Pending& P = ctx->ring[slot];
@@ -2423,7 +2427,6 @@ int cgs_execute_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_composit
   P.W = W;
   P.H = H;
   P.write_f32 = d.write_f32;
-  P.overflowed = false;
   P.cam = *camera;
   P.comp = *comp;
   P.params = *params;
@@ -2812,8 +2815,6 @@ int rerender_slot(cgs_ctx* ctx, int k, uint32_t* out, uint32_t pitch) {
   ctx->deformed_valid = false;
   ctx->s3_valid = false;
   ctx->arena_rerendered = true;
-  p.overflowed = false;
-  ++ctx->rerun_count;
   return rc;
 }
 
@@ -2835,27 +2836,18 @@ int cgs_readback_wait(cgs_ctx* ctx, uint64_t ticket) {
   // (an entry overflow re-renders the latest frame with grown buffers).
   cgs_ctx::Pending& p = ctx->ring[r->frame_slot];
   if (p.used && p.seq == r->frame_seq) CGS_TRY(check_slot(ctx, r->frame_slot, true));
-  // re-rendered after the snapshot, with another frame the last one by now
-  const bool stale = ctx->rerun_count != r->reruns && ctx->rerun_seq == r->frame_seq &&
-                     (ctx->latest_slot < 0 || ctx->ring[ctx->latest_slot].seq != r->frame_seq);
-  if ((p.overflowed || stale) && p.seq == r->frame_seq) {
-    // its entries overflowed while a later frame was in flight, or it was
-    // rendered again before that frame was enqueued: render it again into the
-    // snapshot buffer, then copy that
-    CGS_TRY(rerender_slot(ctx, r->frame_slot, r->stage.as<uint32_t>(), r->W));
-    CGS_CUDA(cudaMemcpyAsync(r->dst, r->stage.p, (size_t)r->W * r->H * 4, cudaMemcpyDeviceToHost,
-                             ctx->stream), "framebuffer readback");
-    CGS_CUDA(cudaStreamSynchronize(ctx->stream), "framebuffer readback");
-    return ctx->take_sticky();
-  }
-  if (ctx->rerun_count != r->reruns && ctx->rerun_seq == r->frame_seq) {
-    // re-rendered after the snapshot: copy again while it is the last frame
-    if (ctx->latest_slot < 0 || ctx->ring[ctx->latest_slot].seq != r->frame_seq)
-      return ctx->fail(CGS_E_CAPACITY,
-                       "the frame was re-rendered after its readback began and is no longer the last frame");
+  if (r->stale && ctx->latest_slot >= 0 && ctx->ring[ctx->latest_slot].seq == r->frame_seq) {
+    // rendered again after the snapshot, and the last frame still
     CGS_CUDA(cudaMemcpy2DAsync(r->dst, (size_t)r->W * 4, ctx->fb_rgba8.p, (size_t)ctx->last_pitch * 4,
                                (size_t)r->W * 4, r->H, cudaMemcpyDeviceToHost, ctx->stream),
              "framebuffer readback");
+    CGS_CUDA(cudaStreamSynchronize(ctx->stream), "framebuffer readback");
+  } else if (r->stale) {
+    // another frame is the last one: render this one (its slot is not reused
+    // before) into the snapshot buffer, then copy that
+    CGS_TRY(rerender_slot(ctx, r->frame_slot, r->stage.as<uint32_t>(), r->W));
+    CGS_CUDA(cudaMemcpyAsync(r->dst, r->stage.p, (size_t)r->W * r->H * 4, cudaMemcpyDeviceToHost,
+                             ctx->stream), "framebuffer readback");
     CGS_CUDA(cudaStreamSynchronize(ctx->stream), "framebuffer readback");
   }
   return ctx->take_sticky();
@@ -2891,7 +2883,7 @@ int cgs_readback_rgba8_async(cgs_ctx* ctx, uint8_t* dst, uint32_t width, uint32_
   r.ticket = t;
   r.frame_slot = ctx->latest_slot;
   r.frame_seq = ctx->ring[ctx->latest_slot].seq;
-  r.reruns = ctx->rerun_count;
+  r.stale = false;
   r.dst = dst;
   r.W = width;
   r.H = height;

@@ -917,7 +917,11 @@ int check_slot(cgs_ctx* ctx, int k, bool block) {
   if (status & kStatusPoisoned) ctx->poisoned = true;
   if (p.stage3_ran && overflowed(h.fc, p.cap)) {
     if (k == ctx->latest_slot) {
-      CGS_TRY(rerun_stage34(ctx));
+      const int rc = rerun_stage34(ctx);
+      if (rc != CGS_OK) {
+        ctx->s3_valid = false;  // the lists are not whole: no later frame may reuse them
+        return rc;
+      }
       entries = ctx->h_ring[k].fc.entries;
     } else {
       // a later frame is in flight: its pixels are rendered again if a

@@ -75,3 +75,30 @@ def test_copy_outlives_its_frames_slot():
         np.testing.assert_array_equal(out, st.readback_framebuffer_rgba8(w, h))
     finally:
         st.close()
+
+
+def test_failed_growth_is_not_reused():
+    """A frame whose lists do not fit the device budget fails; the same frame
+    again fails too instead of reusing what was listed, and renders once the
+    budget allows it."""
+    w, h = 1280, 720
+    scene = random_scene(20_000, seed=4, box=1.0)
+    scene.covariances_3d[:] *= np.float32(100.0)
+    far, near = look(100.0, w, h), look(2.5, w, h)
+    st = GpuPipelineState(0)
+    try:
+        st.upload_scene(scene)
+        comp = compositor(w, h, near, deg=1)
+        st.execute_frame_gpu(scene, None, far, compositor(w, h, far, deg=1), write_f32=True)
+        st.set_device_budget(st.device_bytes() + (64 << 10))
+        for _ in range(3):
+            with pytest.raises(_abi.CgsError) as e:
+                st.execute_frame_gpu(scene, None, near, comp, write_f32=True)
+            assert e.value.code == _abi.CGS_E_OOM
+        st.set_device_budget(0)
+        t = st.execute_frame_gpu(scene, None, near, comp, write_f32=True)
+        o = oracle_frame(scene, near, comp)
+        assert t.total_tile_entries == o["entries"]
+        assert_stage23_exact(gpu_buffers(st), o)
+    finally:
+        st.close()

@@ -2220,11 +2220,12 @@ int enqueue_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_compositor* 
   if (!cached) {
     if (ctx->entry_cap == 0)
       ctx->entry_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(32ull * mn, 1u << 20), (uint64_t)kMaxEntryCap);
-    if (ctx->list_cap == 0)
-      ctx->list_cap = (uint32_t)std::min<uint64_t>((uint64_t)d.total_tiles * kListLimit,
-                                                   std::max<uint64_t>(32ull * mn, 1u << 20));
-    if (ctx->pair_cap == 0)
-      ctx->pair_cap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(4ull * mn, 1u << 16), (uint64_t)kMaxEntryCap);
+    // the lists start from what this viewport and scene may need, also after a
+    // smaller viewport or scene: a frame that does not fit is rendered twice
+    ctx->list_cap = std::max(ctx->list_cap, (uint32_t)std::min<uint64_t>(
+                                                (uint64_t)d.total_tiles * kListLimit, ctx->entry_cap));
+    ctx->pair_cap = std::max(ctx->pair_cap, (uint32_t)std::min<uint64_t>(
+                                                std::max<uint64_t>(4ull * mn, 1u << 16), kMaxEntryCap));
     CGS_TRY(ensure_stage3_buffers(ctx, d));
     if (d.lists) CGS_TRY(ctx->ensure(ctx->list_boxes, (size_t)mn * 4, "splat block boxes"));
     CGS_TRY(ensure_splat_buffers(ctx, mn));

@@ -102,3 +102,69 @@ def test_failed_growth_is_not_reused():
         assert_stage23_exact(gpu_buffers(st), o)
     finally:
         st.close()
+
+
+def test_no_view_twice_after_a_smaller_viewport_or_scene():
+    """A viewport or scene after a smaller one fits where it fits a new context."""
+    def views(st, scene, sizes):
+        cams = [config0_camera(*wh) for wh in sizes]
+        comps = [CompositorUniforms(*wh) for wh in sizes]
+        return st.execute_views(scene, None, cams, comps, st.view_images(comps), use_graph=False)
+
+    st = GpuPipelineState(0)
+    try:
+        scene = random_scene(60_000, seed=6, box=1.0)
+        st.upload_scene(scene)
+        st.upload_cages(None)
+        assert views(st, scene, [(1280, 720)])["views_rerendered"] == 0
+    finally:
+        st.close()
+    st = GpuPipelineState(0)
+    try:
+        st.upload_scene(random_scene(10, seed=6, box=1.0))
+        st.upload_cages(None)
+        views(st, random_scene(10, seed=6, box=1.0), [(16, 16)])
+        st.upload_scene(scene)
+        st.upload_cages(None)
+        assert views(st, scene, [(32, 32), (1280, 720)])["views_rerendered"] == 0
+    finally:
+        st.close()
+
+
+@pytest.mark.parametrize("sort", [_abi.SORT_AUTO, _abi.SORT_RADIX, _abi.SORT_TRANSPOSE])
+def test_overflow_is_listed_again(sort):
+    """Each way to make the lists starts a fresh context with buffers below this
+    frame's needs (2^20 entries, max(4 n, 2^16) pairs of a splat and an 8x4-tile
+    block): the views are rendered again, and a frame equals the oracle."""
+    w, h = 1920, 1080
+    scene = random_scene(4000, seed=13)
+    scene.covariances_3d[:] = np.array([0.09, 0.0, 0.0, 0.09, 0.0, 0.09], np.float32)
+    scene.positions *= np.float32(0.4)
+    cam = config0_camera(w, h)
+    comp = compositor(w, h, cam, deg=1)
+    o = oracle_frame(scene, cam, comp)
+    # the splats' tile boxes from the oracle's extents and centres
+    ext = o["ext"]
+    mu = o["attrs"].reshape(-1, 10)[:, :2]
+    ex, ey = (ext & 0xFFFF).astype(np.float32), (ext >> 16).astype(np.float32)
+    tiles = [np.clip(np.floor(np.stack([mu[:, k] - e, mu[:, k] + e]) / 16), 0, n - 1).astype(np.int64)
+             for k, e, n in ((0, ex, 120), (1, ey, 68))]
+    blocks = np.prod([(t[1] >> s) - (t[0] >> s) + 1 for t, s in zip(tiles, (3, 2))], 0)
+    assert blocks[ext != 0].sum() > 1 << 16 and o["entries"] > 1 << 20
+    st = GpuPipelineState(0)
+    try:
+        st.upload_scene(scene)
+        st.upload_cages(None)
+        images = st.view_images([comp])
+        assert st.execute_views(scene, None, [cam], [comp], images, use_graph=False,
+                                entry_sort=sort)["views_rerendered"] > 0
+        st.close()
+        st = GpuPipelineState(0)
+        st.upload_scene(scene)
+        t = st.execute_frame_gpu(scene, None, cam, comp, force_stage3=True, write_f32=True,
+                                 entry_sort=sort)
+        assert t.total_tile_entries == o["entries"]
+        assert_stage23_exact(gpu_buffers(st), o)
+        assert np.abs(st.readback_framebuffer_f32(w, h) - o["rgba_f32"]).max() <= 2e-3
+    finally:
+        st.close()

@@ -868,6 +868,7 @@ int rerun_stage34(cgs_ctx* ctx) {
   const FrameCounters& f = ctx->h_ring[ctx->latest_slot].fc;
   // the entries are counted once all pairs are held: at most one run more
   for (int attempt = 0; attempt < 3; ++attempt) {
+    if (f.pairs && f.entries > kMaxEntryCap) break;
     grow_caps(ctx, f, 100, 25);
     CGS_TRY(ensure_stage3_buffers(ctx, d));
     // keep fc->surviving and fc->active (Stage 2's words); clear the Stage 3 words

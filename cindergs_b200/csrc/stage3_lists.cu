@@ -401,8 +401,11 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
   __shared__ uint32_t s_delta[kListWarps][32], s_end[kListWarps][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t chunks = a.plan->chunks, groups = a.plan->groups;
-  if (blockIdx.x == 0 && threadIdx.x == 0)
-    a.fc->entries = (uint32_t)min(a.fc->stage_ctr, 0xFFFFFFFFull);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const unsigned long long all = a.fc->stage_ctr;
+    a.fc->entries = (uint32_t)min(all, 0xFFFFFFFFull);
+    if (all > kMaxEntryCap) atomicOr(&a.fc->status, kStatusCapacity);  // as the entry sorts
+  }
   uint16_t* stage = s_stage[warp];
   for (uint32_t c = blockIdx.x * kListWarps + warp; c < chunks; c += gridDim.x * kListWarps) {
     uint32_t rank = a.chunk_base[(size_t)c * 32 + lane];

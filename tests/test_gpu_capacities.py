@@ -168,3 +168,26 @@ def test_overflow_is_listed_again(sort):
         assert np.abs(st.readback_framebuffer_f32(w, h) - o["rgba_f32"]).max() <= 2e-3
     finally:
         st.close()
+
+
+def test_more_entries_than_a_frame_may_have():
+    """More than 2^32 - 2^16 tile entries are refused, however the lists are
+    made: 80,000 splats over 65,536 tiles each."""
+    w, h, n = 7680, 4320, 80_000
+    scene = random_scene(n, seed=3)
+    scene.positions[:] = np.random.default_rng(3).uniform(-0.3, 0.3, (n, 3)).astype(np.float32)
+    scene.covariances_3d[:] = np.array([4.0, 0.0, 0.0, 4.0, 0.0, 4.0], np.float32)
+    scene.opacities[:] = 0.9
+    cam = look(4.0, w, h)
+    st = GpuPipelineState(0)
+    try:
+        st.upload_scene(scene)
+        with pytest.raises(_abi.CgsError) as e:
+            st.execute_frame_gpu(scene, None, cam, compositor(w, h, cam, deg=0), force_stage3=True,
+                                 tile_shape=_abi.TILE_8X8)
+        assert e.value.code == _abi.CGS_E_CAPACITY
+        far = look(60.0, 320, 180)  # the context goes on
+        small = compositor(320, 180, far, deg=0)
+        assert st.execute_frame_gpu(scene, None, far, small, force_stage3=True).total_tile_entries > 0
+    finally:
+        st.close()

@@ -314,7 +314,7 @@ cudaError_t FieldState::backward(uint32_t B, cudaStream_t s) {
   return launch_gemm_grads(gb, s);
 }
 
-cudaError_t FieldState::update(uint32_t B, float lr, cudaStream_t s) {
+cudaError_t FieldState::update(uint32_t B, const float* lr, cudaStream_t s) {
   FieldUpdate u{};
   for (int k = 0; k <= kFieldParams; ++k) u.off[k] = off[k];
   u.V = V;
@@ -328,10 +328,10 @@ cudaError_t FieldState::update(uint32_t B, float lr, cudaStream_t s) {
   u.v = m2.as<float>();
   u.pb = pb.as<__nv_bfloat16>();
   transposed(u.wT);
-  u.adam = lr > 0.0f ? 1 : 0;
+  u.adam = lr ? 1 : 0;
   if (u.adam) {
     ++step;
-    u.lr = lr;
+    u.lr = *lr;
     u.b1 = 0.9f;
     u.b2 = 0.999f;
     u.eps = 1e-8f;

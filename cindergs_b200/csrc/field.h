@@ -69,9 +69,10 @@ struct FieldState {
   cudaError_t forward(const float* points, const float* target, uint32_t n, uint32_t B,
                       uint32_t seed, const float4* rest_verts, float lambda, cudaStream_t s);
   // Products of the backward pass; update() turns their partial sums into the
-  // gradients and, with lr > 0, takes an Adam step.
+  // gradients and, with a learning rate, takes an Adam step (also at a rate
+  // that has underflowed to 0: the moments go on).
   cudaError_t backward(uint32_t B, cudaStream_t s);
-  cudaError_t update(uint32_t B, float lr, cudaStream_t s);
+  cudaError_t update(uint32_t B, const float* lr, cudaStream_t s);
   // bf16 copy (and the transposed weights) from the fp32 parameters
   cudaError_t refresh(cudaStream_t s);
   void transposed(__nv_bfloat16* (&w)[4]) const;

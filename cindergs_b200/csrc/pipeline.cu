@@ -1725,7 +1725,8 @@ int cgs_mvc_field_train(cgs_ctx* ctx, uint64_t n, const float* d_points, const f
                        lambda, s), "field forward");
     CGS_CUDA(f.backward(batch, s), "field backward");
     const double c = 0.5 * (1.0 + std::cos(3.141592653589793 * (double)t / (double)steps));
-    CGS_CUDA(f.update(batch, lr * (float)(0.05 + 0.95 * c), s), "field update");
+    const float lr_t = lr * (float)(0.05 + 0.95 * c);
+    CGS_CUDA(f.update(batch, &lr_t, s), "field update");
   }
   float hl[2] = {0.0f, 0.0f};
   CGS_CUDA(cudaMemcpyAsync(hl, f.loss.p, 8, cudaMemcpyDeviceToHost, s), "field train");
@@ -1749,7 +1750,7 @@ int cgs_mvc_field_grads(cgs_ctx* ctx, uint64_t n, const float* d_points, const f
   CGS_CUDA(f.forward(d_points, d_weights, (uint32_t)n, (uint32_t)n, 0, ctx->mvc_rest.as<float4>(),
                      lambda, s), "field forward");
   CGS_CUDA(f.backward((uint32_t)n, s), "field backward");
-  CGS_CUDA(f.update((uint32_t)n, 0.0f, s), "field gradients");
+  CGS_CUDA(f.update((uint32_t)n, nullptr, s), "field gradients");
   float hl[2];
   CGS_CUDA(cudaMemcpyAsync(hl, f.loss.p, 8, cudaMemcpyDeviceToHost, s), "field grads");
   CGS_TRY(field_status(ctx, "field gradients"));

@@ -487,8 +487,8 @@ struct SortArgs {
   // the widest radix (256), so that a narrow sort leaves no stale word for a
   // later wide one to read.
   uint32_t lb_stride = 0;
-  // 4,096-key tiles whatever the capacity: for callers whose look-back area
-  // does not follow sort_tiles
+  // 4,096-key tiles whatever the capacity: for callers with a line of their own
+  // or a look-back area of a fixed size
   bool large_tiles = false;
   uint32_t* tile_ctr;    // [passes] zeroed
   uint32_t* status_word;
@@ -515,7 +515,7 @@ cudaError_t run_radix_sort(const SortArgs& a, int* out_src, cudaStream_t s);
 cudaError_t launch_histogram(const uint32_t* keys, const uint32_t* n_ptr, uint32_t capacity,
                              uint32_t first_bit, uint32_t num_bits, uint32_t radix_bits,
                              uint32_t* hist, cudaStream_t s);
-uint32_t sort_tiles(uint32_t capacity);  // tiles of a sort without large_tiles
+uint32_t sort_tiles(uint32_t capacity, bool large_tiles = false);  // tiles of a sort
 uint32_t sort_passes(uint32_t num_bits, uint32_t radix_bits);
 
 // ---- Cage springs (springs.cu) -----------------------------------------------

@@ -3415,12 +3415,20 @@ int cgs_scan_u32(cgs_ctx* ctx, const uint32_t* d_in, uint32_t* d_out, uint64_t n
   return CGS_OK;
 }
 
+// Pairs up to which a sort of device arrays takes 2,048-key tiles; beyond,
+// 4,096-key ones. Whole calls with the copies of their inputs, four 8-bit
+// passes of uniform 32-bit keys, 2,048 / 4,096: 20k pairs 69 / 78 us, 300k 86 /
+// 96, 600k 98 / 98, 1M 121 / 111, 1.5M 140 / 122 (equal keys 150 / 133); two
+// words a key, two passes: 300k 155 / 176, 700k 163 / 162, 1M 192 / 172.
+constexpr uint64_t kSortSmallTiles = 5u << 17;
+
 static int sort_common(cgs_ctx* ctx, uint32_t* d_keys, uint32_t* d_vals, uint32_t* d_vals2,
                        uint64_t n, uint32_t key_bits, int32_t digit_bits, int* out_in_scratch,
                        uint32_t** alt) {
   const uint32_t rb = digit_bits == 0 ? 8u : (uint32_t)digit_bits;
   const uint32_t passes = sort_passes(key_bits, rb);
-  const uint32_t stiles = sort_tiles((uint32_t)n);
+  const bool large_tiles = n > kSortSmallTiles;
+  const uint32_t stiles = sort_tiles((uint32_t)n, large_tiles);
   const size_t R = (size_t)1 << rb;
   const size_t hdr = 256 + 8 * 256 * 4;
   const size_t bytes = hdr + (size_t)passes * stiles * R * 4;
@@ -3447,11 +3455,14 @@ static int sort_common(cgs_ctx* ctx, uint32_t* d_keys, uint32_t* d_vals, uint32_
   sa.first_bit = 0;
   sa.num_bits = key_bits;
   // arbitrary keys: a warp's 32 digits are mostly different (48 us a pass of 3M
-  // pairs with one ballot per digit bit)
+  // pairs with one ballot per digit bit); where they are equal, the lanes'
+  // atomics meet in one word, which still costs less than the ballots (8M
+  // pairs: uniform keys 345 us, equal ones 394; 459 and 423 with ballots)
   sa.smem_mask = ~0u;
   sa.radix_bits = rb;
   sa.hist = hist;
   sa.status = b + hdr;
+  sa.large_tiles = large_tiles;
   sa.tile_ctr = words + 2;
   sa.status_word = words + 1;
   sa.src = 0;

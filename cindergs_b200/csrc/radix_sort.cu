@@ -40,13 +40,12 @@ constexpr int kSortWarps = kSortThreads / 32;
 constexpr uint32_t sort_tile_padded(int items) { return kSortThreads * items + kSortThreads * items / 32; }
 // Keys per thread. A tile of 16 keys a thread ranks them one after another and
 // leaves SMs idle below about 148 tiles; one of 8 has twice the blocks and half
-// that chain, but twice the look-back. Measured with 8 / 16 (4) keys a thread:
-// three 8-bit passes of 20k pairs 94 / 97 (93) us with the call around them,
-// of 300k 113 / 122 (121), 600k 121 / 121 (134), 1.2M 139 / 136 (160), 3M 196 /
-// 185 (235); a frame's splat sort, 20k 24 / 31 (24) us, 1.1M in a capacity of
-// 1.4M 55 / 63 (68) us. The line lies where the frame's sorts, whose narrower
-// digits look back less, still gain. It depends on the capacity alone, which
-// the look-back buffers are sized and cleared for.
+// that chain, but twice the look-back. Measured with 8 / 16 (4) keys a thread
+// for a frame's splat sort: 20k slots 24 / 31 (24) us, 1.1M in a capacity of
+// 1.4M 55 / 63 (68). The line lies where the frame's sorts, whose digits are
+// narrow, still gain; sorts of device arrays have another (large_tiles). It
+// depends on the capacity alone, which the look-back buffers are sized and
+// cleared for.
 int sort_items(uint32_t capacity) { return capacity <= 3u << 19 ? 8 : 16; }
 __device__ __forceinline__ uint32_t padded(uint32_t i) { return i + (i >> 5); }
 // Look-back words: a flag (tile count published / inclusive prefix
@@ -419,8 +418,8 @@ cudaError_t launch_drill_digit_lookback(const uint32_t* status, uint32_t radix,
   return cudaGetLastError();
 }
 
-uint32_t sort_tiles(uint32_t capacity) {
-  const uint32_t tile = kSortThreads * sort_items(capacity);
+uint32_t sort_tiles(uint32_t capacity, bool large_tiles) {
+  const uint32_t tile = kSortThreads * (large_tiles ? 16 : sort_items(capacity));
   return (capacity + tile - 1) / tile;
 }
 

@@ -423,6 +423,16 @@ struct ListArgs {
   uint32_t* ids;                // [entry_cap] splat indices, up to kListLimit of every tile
   uint32_t entry_cap;
 };
+// Readback of whole lists in the reference's order: tile by tile over the screen.
+struct ListExport {
+  const uint32_t* tile_at;  // [tiles] first entry of each tile
+  const uint32_t* depths;   // [max_n] depth key of each splat (keys)
+  uint32_t entries;         // of all tiles
+  uint32_t* ids;            // [entries] splat indices, or null
+  void* keys;               // [entries] (tile, depth key), 32 or 64 bits each, or null
+  uint32_t key64, depth_bits;
+  uint32_t* counts;         // [max_n] zeroed: entries of each splat, or null
+};
 // Chunks, ballot groups and placing segments of a frame of at most pair_cap pairs.
 inline uint32_t list_chunk_cap(uint32_t pair_cap, uint32_t blocks) {
   const uint32_t all = pair_cap / 32 + 1, most = kListSmallPairs / 32;
@@ -440,6 +450,10 @@ cudaError_t launch_list_pairs(const ListArgs& a, cudaStream_t s);
 cudaError_t launch_list_count(const ListArgs& a, cudaStream_t s);
 cudaError_t launch_list_place(const ListArgs& a, cudaStream_t s);
 cudaError_t launch_list_write(const ListArgs& a, cudaStream_t s);
+cudaError_t launch_list_export(const ListArgs& a, const ListExport& e, cudaStream_t s);
+// depths[ids[j]] = keys[j] for j < n
+cudaError_t launch_list_depths(const uint32_t* ids, const uint32_t* keys, uint32_t n, uint32_t* depths,
+                               cudaStream_t s);
 
 // Per-tile [start, end) from sorted words: tile = word >> shift, over
 // min(*n_ptr, capacity) words. ranges zeroed.

@@ -2955,8 +2955,8 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
   const size_t active = ctx->last_active;
   const size_t splits = active > ctx->n ? active - ctx->n : 0;
   const size_t entries = ctx->s3_entries;
-  // the screen-block lists keep every block's tiles together: the reference's
-  // order (tile by tile over the screen) is put together here
+  // the screen-block lists keep every block's tiles together; they are read
+  // back in the reference's order, tile by tile over the screen
   const bool lists = ctx->s3_lists;
   std::vector<char> tmp;
   auto fetch = [&](const DevBuf& b, size_t bytes) -> int {
@@ -2966,66 +2966,89 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
     cudaError_t e = cudaMemcpy(tmp.data(), b.p, bytes, cudaMemcpyDeviceToHost);
     return e == cudaSuccess ? CGS_OK : ctx->cuda_fail(e, "buffer readback");
   };
-  // screen-block lists: the splat indices in tile order and the tiles' ranges,
-  // from the blocks' hit words
-  std::vector<uint32_t> l_ids, l_ranges;
-  auto fetch_lists = [&]() -> int {
-    const FrameDesc& d = ctx->last_desc;
-    const ScratchLayout L(d.n, d.max_n ? d.max_n : 1u);
-    const ListLayout B(ctx->list_pairs, ctx->list_blocks);
-    auto words = [&](const DevBuf& buf, size_t off, size_t n, std::vector<uint32_t>* out) -> int {
-      out->resize(n);
-      if (n == 0) return CGS_OK;
-      if (!buf.p || buf.cap < off + n * 4) return ctx->fail(CGS_E_STATE, "buffer not populated by the last frame");
-      const cudaError_t e = cudaMemcpy(out->data(), buf.as<char>() + off, n * 4, cudaMemcpyDeviceToHost);
-      return e == cudaSuccess ? CGS_OK : ctx->cuda_fail(e, "buffer readback");
-    };
-    std::vector<uint32_t> start, chunk, masks, pairs;
-    CGS_TRY(words(ctx->scratch, L.lstart, d.num_blocks + 1, &start));
-    CGS_TRY(words(ctx->scratch, L.lchunk, d.num_blocks + 1, &chunk));
-    const uint32_t np = start[d.num_blocks], groups = np <= kListSmallPairs ? 1u : kListGroups;
-    CGS_TRY(words(ctx->lists, B.masks, (size_t)chunk[d.num_blocks] * groups * 32, &masks));
-    CGS_TRY(words(ctx->lists, B.ids[ctx->list_src], np, &pairs));
-    // every (tile, first pair, word) in block and pair order, twice: counts, then places
-    std::vector<uint32_t> at(d.total_tiles, 0);
-    auto walk = [&](auto&& fn) {
-      for (uint32_t b = 0; b < d.num_blocks; ++b)
-        for (uint32_t k = 0; k < (chunk[b + 1] - chunk[b]) * groups; ++k) {
-          const uint32_t i0 = start[b] + 32 * k;
-          if (i0 >= start[b + 1]) continue;
-          for (uint32_t t = 0; t < 32; ++t) {
-            const uint32_t tx = ((b % d.blocks_x) << kListBlockW) + (t & 7u);
-            const uint32_t ty = ((b / d.blocks_x) << kListBlockH) + (t >> 3);
-            const uint32_t m = masks[((size_t)chunk[b] * groups + k) * 32 + t];
-            if (m && tx < d.tiles_x && ty < d.tiles_y) fn(ty * d.tiles_x + tx, i0, m);
-          }
-        }
-    };
-    walk([&](uint32_t tile, uint32_t, uint32_t m) { at[tile] += (uint32_t)__builtin_popcount(m); });
-    l_ranges.assign(2 * (size_t)d.total_tiles, 0);
-    uint32_t run = 0;
-    for (uint32_t t = 0; t < d.total_tiles; ++t) {
-      if (at[t]) {
-        l_ranges[2 * (size_t)t] = run;
-        l_ranges[2 * (size_t)t + 1] = run + at[t];
+  std::vector<char> out;
+  // screen-block lists: the tiles' ranges in the reference's order, from their
+  // counts; the entries and the splats' counts from the blocks' hit words
+  std::vector<uint32_t> l_ranges;
+  auto list_ranges = [&]() -> int {
+    const uint32_t tiles = ctx->last_desc.total_tiles;
+    CGS_TRY(fetch(ctx->ranges, (size_t)tiles * 8));
+    const uint32_t* r = (const uint32_t*)tmp.data();
+    l_ranges.assign(2 * (size_t)tiles, 0);
+    uint64_t run = 0;
+    for (size_t t = 0; t < tiles; ++t) {
+      const uint32_t n = r[2 * t + 1];
+      if (n) {
+        l_ranges[2 * t] = (uint32_t)run;
+        l_ranges[2 * t + 1] = (uint32_t)(run + n);
       }
-      const uint32_t n = at[t];
-      at[t] = run;
       run += n;
     }
-    if (run != entries) return ctx->fail(CGS_E_STATE, "the lists' words and the entry total differ");
-    l_ids.resize(run);
-    walk([&](uint32_t tile, uint32_t i0, uint32_t m) {
-      for (; m; m &= m - 1) l_ids[at[tile]++] = pairs[i0 + (uint32_t)__builtin_ctz(m)];
-    });
+    if (run != entries) return ctx->fail(CGS_E_STATE, "the tiles' counts and the entry total differ");
     return CGS_OK;
   };
-  auto bytes_of = [](const std::vector<uint32_t>& v) {
-    std::vector<char> b(v.size() * 4);
-    std::memcpy(b.data(), v.data(), b.size());
-    return b;
+  // ids, keys or per-splat counts (by `which`) into out
+  auto export_lists = [&]() -> int {
+    CGS_TRY(list_ranges());
+    const FrameDesc& d = ctx->last_desc;
+    cudaStream_t s = ctx->stream;
+    const bool keys = which == CGS_BUF_SORTED_KEYS, counts = which == CGS_BUF_TILE_OFFSETS;
+    const bool k64 = ctx->s3_key64 != 0;
+    const size_t items = counts ? ctx->s3_active : entries, bytes = items * (keys && k64 ? 8 : 4);
+    out.resize(bytes);
+    if (bytes == 0 || !dst) return CGS_OK;
+    const ScratchLayout L(d.n, d.max_n ? d.max_n : 1u);
+    const ListLayout B(ctx->list_pairs, ctx->list_blocks);
+    if (!ctx->lists.p || !ctx->scratch.p) return ctx->fail(CGS_E_STATE, "buffer not populated by the last frame");
+    const char* lp = ctx->lists.as<char>();
+    const char* sc = ctx->scratch.as<char>();
+    std::vector<uint32_t> at(d.total_tiles);
+    for (size_t t = 0; t < at.size(); ++t) at[t] = l_ranges[2 * t];
+    const size_t mn = d.max_n ? d.max_n : 1;
+    DevBuf places, result, depths;
+    if (cudaMalloc(&places.p, at.size() * 4) != cudaSuccess ||
+        cudaMalloc(&result.p, counts ? mn * 4 : bytes) != cudaSuccess ||
+        (keys && cudaMalloc(&depths.p, mn * 4) != cudaSuccess)) {
+      cudaGetLastError();
+      return ctx->fail(CGS_E_OOM, "device allocation failed for the readback of the tile lists");
+    }
+    ListArgs a{};
+    a.max_n = d.max_n;
+    a.tiles_x = d.tiles_x;
+    a.tiles_y = d.tiles_y;
+    a.blocks_x = d.blocks_x;
+    a.num_blocks = d.num_blocks;
+    a.block_start = (uint32_t*)(sc + L.lstart);
+    a.chunk_first = (uint32_t*)(sc + L.lchunk);
+    a.pair_cap = ctx->list_pairs;
+    a.masks = (uint32_t*)(lp + B.masks);
+    a.chunk_base = (uint32_t*)(lp + B.base);
+    a.sorted_pairs = (const uint32_t*)(lp + B.ids[ctx->list_src]);
+    ListExport e{};
+    e.tile_at = places.as<uint32_t>();
+    e.entries = (uint32_t)entries;
+    e.key64 = k64;
+    e.depth_bits = ctx->s3_depth_bits;
+    CGS_CUDA(cudaMemcpyAsync(places.p, at.data(), at.size() * 4, cudaMemcpyHostToDevice, s), "buffer readback");
+    if (counts) {
+      e.counts = result.as<uint32_t>();
+      CGS_CUDA(cudaMemsetAsync(result.p, 0, mn * 4, s), "buffer readback");
+    } else if (keys) {
+      e.keys = result.p;
+      e.depths = depths.as<uint32_t>();
+      CGS_CUDA(cudaMemsetAsync(depths.p, 0, mn * 4, s), "buffer readback");
+      CGS_CUDA(launch_list_depths(ctx->sids[ctx->s3_order_src].as<uint32_t>(),
+                                  ctx->skeys[ctx->s3_order_src].as<uint32_t>(),
+                                  std::min(ctx->s3_active, d.max_n), depths.as<uint32_t>(), s),
+               "buffer readback");
+    } else {
+      e.ids = result.as<uint32_t>();
+    }
+    CGS_CUDA(launch_list_export(a, e, s), "buffer readback");
+    CGS_CUDA(cudaMemcpyAsync(out.data(), result.p, bytes, cudaMemcpyDeviceToHost, s), "buffer readback");
+    CGS_CUDA(cudaStreamSynchronize(s), "buffer readback");
+    return CGS_OK;
   };
-  std::vector<char> out;
   switch (which) {
     case CGS_BUF_DEFORMED_POS:
     case CGS_BUF_DEFORMED_OPA: {
@@ -3091,20 +3114,15 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
       // offsets, the splat order and the entry total.
       const size_t sa = ctx->s3_active;
       if (lists) {
-        // a splat's count is its number of entries
-        CGS_TRY(fetch_lists());
-        std::vector<uint32_t> cnt(sa, 0);
-        for (uint32_t id : l_ids) {
-          if (id >= sa) return ctx->fail(CGS_E_STATE, "splat index out of range");
-          ++cnt[id];
-        }
+        // scan of the splats' entry counts
+        CGS_TRY(export_lists());
+        uint32_t* o = (uint32_t*)out.data();
         uint32_t run = 0;
-        for (uint32_t& c : cnt) {
-          const uint32_t n = c;
-          c = run;
+        for (size_t i = 0; i < sa; ++i) {
+          const uint32_t n = o[i];
+          o[i] = run;
           run += n;
         }
-        out = bytes_of(cnt);
         break;
       }
       CGS_TRY(fetch(ctx->offsets, sa * 4));
@@ -3129,28 +3147,7 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
     }
     case CGS_BUF_SORTED_KEYS:
       if (lists) {
-        // (tile, depth) of every entry from the ranges and the splats' depth keys
-        const size_t sa = ctx->s3_active;
-        CGS_TRY(fetch_lists());
-        CGS_TRY(fetch(ctx->sids[ctx->s3_order_src], sa * 4));
-        const std::vector<char> ord = tmp;
-        CGS_TRY(fetch(ctx->skeys[ctx->s3_order_src], sa * 4));
-        const uint32_t* os = (const uint32_t*)ord.data();
-        const uint32_t* ds = (const uint32_t*)tmp.data();
-        std::vector<uint32_t> depth(sa, 0);
-        for (size_t j = 0; j < sa; ++j)
-          if (os[j] < sa) depth[os[j]] = ds[j];
-        const bool k64 = ctx->s3_key64 != 0;
-        const uint32_t db = ctx->s3_depth_bits;
-        out.assign(l_ids.size() * (k64 ? 8 : 4), 0);
-        for (uint32_t t = 0; t < ctx->last_tiles; ++t)
-          for (uint32_t i = l_ranges[2 * t]; i < l_ranges[2 * t + 1]; ++i) {
-            const uint32_t dk = l_ids[i] < sa ? depth[l_ids[i]] : 0u;
-            if (k64)
-              ((uint64_t*)out.data())[i] = ((uint64_t)t << 32) | dk;
-            else
-              ((uint32_t*)out.data())[i] = (db >= 32 ? 0u : (t << db)) | dk;
-          }
+        CGS_TRY(export_lists());
       } else if (ctx->s3_transpose) {
         // The tile transpose sorts splat indices only; the 32-bit keys are
         // tile << depth_bits | depth key, from the ranges and the splat order.
@@ -3190,8 +3187,7 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
       break;
     case CGS_BUF_SORTED_IDS:
       if (lists) {
-        CGS_TRY(fetch_lists());
-        out = bytes_of(l_ids);
+        CGS_TRY(export_lists());
         break;
       }
       CGS_TRY(fetch(ctx->ids[ctx->s3_src], entries * 4));
@@ -3199,8 +3195,9 @@ int cgs_read_frame_buffer(cgs_ctx* ctx, int32_t which, void* dst, uint64_t dst_b
       break;
     case CGS_BUF_TILE_RANGES:
       if (lists) {
-        CGS_TRY(fetch_lists());
-        out = bytes_of(l_ranges);
+        CGS_TRY(list_ranges());
+        out.resize(l_ranges.size() * 4);
+        std::memcpy(out.data(), l_ranges.data(), out.size());
         break;
       }
       CGS_TRY(fetch(ctx->ranges, (size_t)ctx->last_tiles * 8));

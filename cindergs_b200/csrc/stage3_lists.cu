@@ -459,6 +459,55 @@ __global__ void __launch_bounds__(kListThreads) k_list_write(const ListArgs a) {
   }
 }
 
+// Every entry of every tile at its place in the reference's order, and how
+// many entries each splat has, from the blocks' hit words: a warp per chunk, a
+// lane per tile. For readbacks only (26M entries put together on the host took
+// 160 ms).
+__global__ void __launch_bounds__(kListThreads) k_list_export(const ListArgs a, const ListExport e) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t chunks = a.chunk_first[a.num_blocks];
+  const uint32_t groups = a.block_start[a.num_blocks] <= kListSmallPairs ? 1u : kListGroups;
+  for (uint32_t c = blockIdx.x * kListWarps + warp; c < chunks; c += gridDim.x * kListWarps) {
+    const uint32_t b = block_of(a.chunk_first, a.num_blocks, c);
+    const uint32_t tx = ((b % a.blocks_x) << kListBlockW) + (lane & 7u);
+    const uint32_t ty = ((b / a.blocks_x) << kListBlockH) + (lane >> 3);
+    const bool on = tx < a.tiles_x && ty < a.tiles_y;
+    const uint32_t tile = ty * a.tiles_x + tx;
+    const uint32_t i0 = a.block_start[b] + (c - a.chunk_first[b]) * 32u * groups;
+    const uint32_t end = min(a.block_start[b + 1], a.pair_cap);
+    uint32_t at = on ? e.tile_at[tile] + a.chunk_base[(size_t)c * 32 + lane] : 0u;
+    for (uint32_t j = 0; j < groups && i0 + 32u * j < end; ++j) {
+      const uint32_t i = i0 + 32u * j;
+      uint32_t m = on ? a.masks[((size_t)c * groups + j) * 32 + lane] : 0u;
+      if (e.counts) {
+        const uint32_t tiles = __popc(transpose_bits(m, lane));  // of pair i + lane
+        const uint32_t sid = i + lane < end ? a.sorted_pairs[i + lane] : kInvalid;
+        if (tiles && sid < a.max_n) atomicAdd(&e.counts[sid], tiles);
+      }
+      if (!e.ids && !e.keys) continue;
+      for (; m; m &= m - 1u, ++at) {
+        if (at >= e.entries) break;
+        const uint32_t sid = a.sorted_pairs[i + (uint32_t)__ffs(m) - 1u];
+        if (e.ids) e.ids[at] = sid;
+        if (e.keys) {
+          const uint32_t d = sid < a.max_n ? e.depths[sid] : 0u;
+          if (e.key64)
+            static_cast<unsigned long long*>(e.keys)[at] = ((unsigned long long)tile << 32) | d;
+          else
+            static_cast<uint32_t*>(e.keys)[at] = (e.depth_bits >= 32u ? 0u : tile << e.depth_bits) | d;
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+__global__ void k_list_depths(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ keys,
+                              uint32_t n, uint32_t* __restrict__ depths) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n && ids[j] < n) depths[ids[j]] = keys[j];
+}
+
 // Resident blocks of kernel K on the current device.
 template <typename K>
 uint32_t resident_blocks(K kernel, int threads) {
@@ -471,6 +520,20 @@ uint32_t resident_blocks(K kernel, int threads) {
 }
 
 }  // namespace
+
+cudaError_t launch_list_export(const ListArgs& a, const ListExport& e, cudaStream_t s) {
+  static const uint32_t grid = resident_blocks(k_list_export, kListThreads);
+  const uint32_t most = (list_chunk_cap(a.pair_cap, a.num_blocks) + kListWarps - 1) / kListWarps;
+  k_list_export<<<std::min(most, grid), kListThreads, 0, s>>>(a, e);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_list_depths(const uint32_t* ids, const uint32_t* keys, uint32_t n, uint32_t* depths,
+                               cudaStream_t s) {
+  if (n == 0) return cudaSuccess;
+  k_list_depths<<<(n + 255) / 256, 256, 0, s>>>(ids, keys, n, depths);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_list_pairs(const ListArgs& a, cudaStream_t s) {
   if (a.num_blocks == 0 || a.num_blocks > kListMaxBlocks) return cudaErrorInvalidValue;

@@ -105,10 +105,11 @@ __device__ __forceinline__ void mvc_eval(const MvcCage& c, F3 x, const EvalSmem&
   __syncthreads();
   const uint32_t fhit = s.hit[1];
   const bool regular = vhit == kNone && fhit == kNone;
-  if (tid == 0 && regular) {
+  if (tid == (int)blockDim.x - 32 && regular) {
     // the normaliser, face by face as the reference accumulates it: one
     // addition per face (the face's own sum is its fourth word), while the
-    // other warps sum their vertices' faces below
+    // other warps sum their vertices' faces below (the last warp has the
+    // fewest, none in a small cage)
     float total = 0.0f;
 #pragma unroll 16
     for (uint32_t f = 0; f < c.F; ++f) total += s.mu[f].w;
@@ -173,9 +174,9 @@ __device__ __forceinline__ EvalSmem eval_smem(unsigned char* base, const MvcCage
 }
 
 // Exact weights of arbitrary points: w[i * V + j]. Bound by the latency of its
-// transcendental functions: six blocks per SM (84 registers) instead of five
-// take 20,011 points against 642 vertices from 890 to 824 us; seven gain
-// nothing more.
+// transcendental functions: asked for six blocks per SM, the compiler takes 63
+// registers (95 before, five blocks), and 20,011 points against 642 vertices
+// take 824 us instead of 890; asked for seven, it gains nothing more.
 __global__ void __launch_bounds__(kMvcThreads, 6) k_mvc_weights(const MvcCage c, uint32_t n,
                                                             const float* __restrict__ pts,
                                                             float* __restrict__ w) {
@@ -195,7 +196,10 @@ __global__ void __launch_bounds__(kMvcThreads, 6) k_mvc_weights(const MvcCage c,
 
 // bind_gaussians (mvc.rs:498-541) for the bound Gaussians: weights and
 // central-difference gradients, stored vertex-major, wg[j * nb + slot] =
-// (w, dw/dx, dw/dy, dw/dz).
+// (w, dw/dx, dw/dy, dw/dz). Bound by the latency of the evaluations' functions.
+// The seven evaluations share one copy of their code: seven copies took longer,
+// probably to fetch (20,000 Gaussians, whole calls: 42 vertices 1.56 -> 0.88 ms,
+// 162 vertices 2.58 -> 2.08, 642 vertices 7.28 -> 6.86).
 __global__ void __launch_bounds__(kMvcThreads, 1) k_mvc_bind_weights(const MvcCage c, uint32_t nb,
                                                                  const uint32_t* __restrict__ list,
                                                                  const float4* __restrict__ rest_pos,
@@ -206,18 +210,27 @@ __global__ void __launch_bounds__(kMvcThreads, 1) k_mvc_bind_weights(const MvcCa
   const float inv_2h = 0.5f / h;
   for (uint32_t slot = blockIdx.x; slot < nb; slot += gridDim.x) {
     const float4 p = rest_pos[list[slot]];
-    float w0[kMaxOwn], wp[kMaxOwn], wm[kMaxOwn], g[3][kMaxOwn];
-    mvc_eval<kMaxOwn>(c, {p.x, p.y, p.z}, s, w0);
+    float w0[kMaxOwn], wp[kMaxOwn], g[3][kMaxOwn];
 #pragma unroll
-    for (int axis = 0; axis < 3; ++axis) {
-      F3 xp = {p.x, p.y, p.z}, xm = {p.x, p.y, p.z};
-      if (axis == 0) { xp.x += h; xm.x -= h; }
-      if (axis == 1) { xp.y += h; xm.y -= h; }
-      if (axis == 2) { xp.z += h; xm.z -= h; }
-      mvc_eval<kMaxOwn>(c, xp, s, wp);
-      mvc_eval<kMaxOwn>(c, xm, s, wm);
+    for (int k = 0; k < kMaxOwn; ++k) w0[k] = wp[k] = g[0][k] = g[1][k] = g[2][k] = 0.0f;
+#pragma unroll 1
+    for (int e = 0; e < 7; ++e) {
+      F3 x = {p.x, p.y, p.z};
+      const float d = (e & 1) ? h : -h;
+      if (e == 1 || e == 2) x.x += d;
+      if (e == 3 || e == 4) x.y += d;
+      if (e >= 5) x.z += d;
+      float we[kMaxOwn];
+      mvc_eval<kMaxOwn>(c, x, s, we);
 #pragma unroll
-      for (int k = 0; k < kMaxOwn; ++k) g[axis][k] = (wp[k] - wm[k]) * inv_2h;
+      for (int k = 0; k < kMaxOwn; ++k) {
+        const float q = (wp[k] - we[k]) * inv_2h;
+        if (e == 0) w0[k] = we[k];
+        if (e == 2) g[0][k] = q;
+        if (e == 4) g[1][k] = q;
+        if (e == 6) g[2][k] = q;
+        wp[k] = we[k];
+      }
     }
 #pragma unroll
     for (int k = 0; k < kMaxOwn; ++k) {

@@ -104,6 +104,9 @@ extern "C" int cgs_sort_pairs_u32_noalloc(uint32_t* d_keys, uint32_t* d_vals, ui
   sa.hist = hist;
   sa.status = status;
   sa.large_tiles = true;  // what kStatusBytes holds
+  // arbitrary keys, as in cgs_sort_pairs_u32: 2^20 uniform pairs 113 -> 97 us
+  // against one ballot per digit bit, equal ones 106 either way
+  sa.smem_mask = ~0u;
   sa.tile_ctr = words + 2;
   sa.status_word = words + 1;
   sa.src = 0;

@@ -608,6 +608,9 @@ struct CompositeArgs {
   const uint32_t* block_start;
   const uint32_t* sorted_pairs;
   uint32_t blocks_x, num_blocks;
+  // set by launch_composite: a pixel without entries
+  uint32_t bg_rgba8;
+  float4 bg_f32;
 };
 cudaError_t launch_composite(const CompositeArgs& a, cudaStream_t s);
 

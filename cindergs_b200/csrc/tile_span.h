@@ -38,6 +38,8 @@ namespace cgs {
 CGS_SPAN_HD float span_rsqrt(float x) {
 #ifdef __CUDA_ARCH__
   return rsqrtf(x);
+#elif defined(CGS_SPAN_RSQRT)
+  return CGS_SPAN_RSQRT(x);  // a test's root with the device function's error
 #else
   return 1.0f / sqrtf(x);
 #endif

@@ -223,7 +223,8 @@ def config_dict(args, wl, world):
     return {"workload": "tet-cage deform + render, orbit camera",
             "gaussians": wl.scene.count, "width": args.width, "height": args.height,
             "cage": "5x5x5 cubes x 6 tets (750 tets, 216 vertices), springs k=40 c=4 dt=1/60",
-            "sh_degree": 3, "keys": "32-bit tile|depth",
+            "sh_degree": 3,
+            "keys": "32-bit tile|depth" if args.entry_sort else "splat depths, block ids of pairs",
             "radix_digits": radix_digits(args) if args.entry_sort == 1 else None,
             "entry_sort": ["auto (screen-block lists)", "radix", "tile transpose"][args.entry_sort],
             "tile": ["16x16", "8x8", "32x16"][args.tile_shape],

@@ -745,6 +745,11 @@ cudaError_t launch_field_loss(const FieldLoss& l, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     return launch_dependent(kernel, (l.B + kLossRows - 1) / kLossRows, 32 * kLossRows, smem, s, l);
   };
+  // A lane holds a 32nd of the columns. The lines lie at the multiples of 32
+  // next above the icospheres of two and three subdivisions (162 and 642
+  // vertices), the larger cages that the presets make; any other size takes the
+  // next larger kernel. Lines every 256 columns took 1 to 4% more a training step
+  // there (162 vertices, 8 steps of 4,096 rows: 985 -> 1,022 us).
   if (l.V <= 192u) return run(k_field_loss<6>);
   if (l.V <= 672u) return run(k_field_loss<21>);
   return run(k_field_loss<32>);

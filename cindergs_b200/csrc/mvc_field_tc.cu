@@ -749,7 +749,7 @@ __global__ void __launch_bounds__(kGmThreads) k_gemm_tc(GemmArgs g) {
 }
 
 // Column sums over the rows of in [B][ld], 32 columns per block, each column's
-// rows added one after the other in row order: the ring of 64-row stages is
+// rows added one after the other in row order: the ring of 128-row stages is
 // filled by the whole block with cp.async while warp 0 adds (4 cycles a row;
 // one thread per column that walked the rows in memory took 160 us at 4,096
 // rows).

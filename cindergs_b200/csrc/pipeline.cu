@@ -612,14 +612,16 @@ int enqueue_lists(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, uint
   return CGS_OK;
 }
 
-// Enqueues Stage 3 for `d` with the current key-buffer capacity:
+// Enqueues Stage 3 for `d` with the current capacities:
 //   1. stable radix sort of Stage 2's per-splat depth keys (skipped with
 //      `sort_splats` false: a re-run of the same frame reuses its order);
-//   2. binning in that order (k_bin): entries leave ordered by depth;
-//   3. stable radix sort of the entries on their tile bits only;
+//   2. the screen-block lists in that order (enqueue_lists), or
+//   2. binning in that order (k_bin_direct): entries leave ordered by depth;
+//   3. stable sort of the entries by tile: radix passes over the tile bits, or
+//      the one-pass tile transpose;
 //   4. tile ranges.
 // *result_src receives the buffer holding the sorted lists; *passes and
-// *splat_passes the number of radix passes over entries and splats.
+// *splat_passes the number of radix passes over pairs or entries and splats.
 int enqueue_stage3(cgs_ctx* ctx, const FrameDesc& d, const ScratchLayout& L, int* result_src,
                    uint32_t* passes, uint32_t* splat_passes, bool sort_splats,
                    uint32_t* bin_launches = nullptr, uint32_t* sort_launches = nullptr) {
@@ -2073,8 +2075,15 @@ bool tile_shape_log2(int32_t shape, uint32_t* lw, uint32_t* lh) {
 
 // Stage 3 goes through the screen-block lists unless the caller names one of
 // the entry sorts, or the viewport has more blocks than the pairing kernel
-// counts in shared memory. Both give the same lists; the lists took 0.28 ms
-// against 0.78 at 26M entries (1080p) and are never behind.
+// counts in shared memory. Both give the same lists, so the line is one of
+// time, drawn for frames of ordinary density, where the lists gain most:
+// Stage 3 of 26M entries (1080p) 0.28 ms against 0.78 by radix passes, whole
+// frames of 20,000 splats at 1080p 158 / 179 us, of 1.5M at 8K 2.1 / 20.3 ms.
+// Radix passes take less where there is little to bin (64x64 pixels: 1 splat
+// 163 / 174 us, 100 splats 167 / 181) and where the lists of few tiles run far
+// past kListLimit entries (16x16 tiles, 320x180: 100,000 splats 522 / 670 us, 1M
+// 2.3 / 3.1 ms; 32x16 tiles, 1M 9.3 / 30.6): neither is known before the frame,
+// and entry_sort or the autotuner chooses them.
 void set_lists(FrameDesc* d) {
   d->blocks_x = (d->tiles_x + (1u << kListBlockW) - 1) >> kListBlockW;
   const uint64_t blocks = (uint64_t)d->blocks_x * ((d->tiles_y + (1u << kListBlockH) - 1) >> kListBlockH);

@@ -1,7 +1,9 @@
-// The pieces of the ellipse-vs-tile test that the binning kernels share
-// (ellipse_intersects_tile_gpu, render/kernels/binning.rs:37-96): the splat's
-// tile box and the column and row terms of a tile, every product and sum
-// rounded separately in the reference's operand order.
+// The pieces of the ellipse-vs-tile test (ellipse_intersects_tile_gpu,
+// render/kernels/binning.rs:37-96), every product and sum rounded separately
+// in the reference's operand order: the splat's tile box and the pixel centres,
+// which the projection, the entry binning and the screen-block lists share, and
+// the column and row terms of a tile with their divisions, for the entry
+// binning.
 #pragma once
 #include "kernels.h"
 

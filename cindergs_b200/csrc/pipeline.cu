@@ -2091,6 +2091,30 @@ void set_lists(FrameDesc* d) {
   d->num_blocks = d->lists ? (uint32_t)blocks : 0u;
 }
 
+// What a frame's viewport and parameters (validated by the caller) make of
+// Stage 3: its tiles, key and digit widths, and the way it takes.
+void set_stage3(FrameDesc* d, uint32_t W, uint32_t H, const cgs_frame_params* params) {
+  tile_shape_log2(params->tile_shape, &d->tile_lw, &d->tile_lh);
+  d->W = W;
+  d->H = H;
+  d->tiles_x = (W + (1u << d->tile_lw) - 1) >> d->tile_lw;
+  d->tiles_y = (H + (1u << d->tile_lh) - 1) >> d->tile_lh;
+  d->total_tiles = (uint32_t)((uint64_t)d->tiles_x * d->tiles_y);
+  d->radix_bits = (uint32_t)params->radix_bits;
+  d->entry_sort = params->entry_sort;
+  d->key64 = d->total_tiles > 65535u;
+  d->tile_bits = d->total_tiles <= 1 ? 1u : 32u - (uint32_t)__builtin_clz(d->total_tiles - 1);
+  d->depth_bits = d->tile_bits >= 32 ? 0u : (32u - d->tile_bits < 28u ? 32u - d->tile_bits : 28u);
+  d->sort_bits = d->tile_bits + d->depth_bits > 32 ? 32 : d->tile_bits + d->depth_bits;
+  if (d->radix_bits == 0) {
+    // balanced digits: the fewest passes of at most 8 bits over the tile bits,
+    // split as evenly as possible (13 bits -> 7 + 6), at least 4 bits
+    const uint32_t passes = (d->tile_bits + 7) / 8;
+    d->radix_bits = std::max(4u, (d->tile_bits + passes - 1) / passes);
+  }
+  set_lists(d);
+}
+
 // How a frame is enqueued (cgs_execute_frame, cgs_execute_views).
 struct FrameCtl {
   bool allow_cache = true;     // may reuse the cached Stage 3 lists
@@ -2138,18 +2162,8 @@ int enqueue_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_compositor* 
   const uint32_t W = comp->screen_width ? comp->screen_width : 1u;
   const uint32_t H = comp->screen_height ? comp->screen_height : 1u;
   FrameDesc d;
-  tile_shape_log2(params->tile_shape, &d.tile_lw, &d.tile_lh);  // validated by the caller
-  const uint32_t tiles_x = (W + (1u << d.tile_lw) - 1) >> d.tile_lw;
-  const uint32_t tiles_y = (H + (1u << d.tile_lh) - 1) >> d.tile_lh;
-  const uint64_t total_tiles64 = (uint64_t)tiles_x * tiles_y;
-  d.W = W;
-  d.H = H;
-  d.tiles_x = tiles_x;
-  d.tiles_y = tiles_y;
-  d.total_tiles = (uint32_t)total_tiles64;
+  set_stage3(&d, W, H, params);
   d.pitch = (W + 63) / 64 * 64;
-  d.radix_bits = (uint32_t)params->radix_bits;
-  d.entry_sort = params->entry_sort;
   d.write_f32 = params->write_f32 != 0;
   std::memcpy(d.bg, comp->background, 16);
   if (W != ctx->last_w || H != ctx->last_h) ctx->s3_valid = false;
@@ -2173,17 +2187,6 @@ int enqueue_frame(cgs_ctx* ctx, const cgs_camera* camera, const cgs_compositor* 
   d.split_possible = deform_on && params->strain_split_threshold > 0.0f;
   d.max_n = d.split_possible ? 2 * n : n;
   const uint32_t mn = d.max_n ? d.max_n : 1u;
-  d.key64 = d.total_tiles > 65535u;
-  d.tile_bits = d.total_tiles <= 1 ? 1u : 32u - (uint32_t)__builtin_clz(d.total_tiles - 1);
-  d.depth_bits = d.tile_bits >= 32 ? 0u : (32u - d.tile_bits < 28u ? 32u - d.tile_bits : 28u);
-  d.sort_bits = d.tile_bits + d.depth_bits > 32 ? 32 : d.tile_bits + d.depth_bits;
-  if (d.radix_bits == 0) {
-    // balanced digits: the fewest passes of at most 8 bits over the tile bits,
-    // split as evenly as possible (13 bits -> 7 + 6), at least 4 bits
-    const uint32_t passes = (d.tile_bits + 7) / 8;
-    d.radix_bits = std::max(4u, (d.tile_bits + passes - 1) / passes);
-  }
-  set_lists(&d);
   const float near_c = camera->near_plane > 1e-6f ? camera->near_plane : 1e-6f;
   d.depth_base_bits = fbits(near_c) & 0x7F800000u;
 
@@ -2620,6 +2623,7 @@ int capture_views(cgs_ctx* ctx, uint32_t nv, const cgs_camera* cams, const cgs_c
   ctx->views_splat_parity = ctx->splat_parity;
   ctx->views_pair_parity = ctx->pair_parity;
   if (rc != CGS_OK || e != cudaSuccess) {
+    cudaGetLastError();  // of the capture: not for the next launch's check to find
     ctx->views_exec = nullptr;
     return rc != CGS_OK ? rc : ctx->cuda_fail(e, "views capture");
   }
@@ -2714,26 +2718,14 @@ int cgs_execute_views(cgs_ctx* ctx, uint32_t num_views, const cgs_camera* camera
                         &st.total_tile_entries));
     CGS_CUDA(cudaEventRecord(ctx->views_ev[1], s), "views event");
     if (use_graph) {
-      // grow the buffers to the capacities the graph will be captured with
-      bool key64 = false, entries = false;
+      // grow the buffers to the capacities the graph will be captured with, for
+      // every view: its key and digit widths are its own
       for (uint32_t v = 0; v < num_views; ++v) {
         FrameDesc d;
-        tile_shape_log2(prm[v].tile_shape, &d.tile_lw, &d.tile_lh);
-        const uint32_t W = comps[v].screen_width ? comps[v].screen_width : 1u;
-        const uint32_t H = comps[v].screen_height ? comps[v].screen_height : 1u;
-        d.tiles_x = (W + (1u << d.tile_lw) - 1) >> d.tile_lw;
-        d.tiles_y = (H + (1u << d.tile_lh) - 1) >> d.tile_lh;
-        d.entry_sort = prm[v].entry_sort;
-        set_lists(&d);
-        if (d.lists) {
-          CGS_TRY(ensure_stage3_buffers(ctx, d));
-          continue;
-        }
-        entries = true;
-        key64 = key64 || (uint64_t)d.tiles_x * d.tiles_y > 65535u;
+        set_stage3(&d, comps[v].screen_width ? comps[v].screen_width : 1u,
+                   comps[v].screen_height ? comps[v].screen_height : 1u, &prm[v]);
+        CGS_TRY(ensure_stage3_buffers(ctx, d));
       }
-      if (entries)
-        CGS_TRY(ensure_entry_buffers(ctx, ctx->entry_cap, key64, ctx->radix_lb_bits ? ctx->radix_lb_bits : 8));
       CGS_TRY(capture_views(ctx, num_views, cameras, comps, prm.data(), d_rgba8));
       ctx->views_key = key_of();
       st.graph_captured = 1;

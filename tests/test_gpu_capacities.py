@@ -4,7 +4,8 @@ import numpy as np
 import pytest
 import torch
 
-from cindergs_b200 import CameraUniforms, CompositorUniforms, GpuPipelineState, _abi, random_scene
+from cindergs_b200 import (CameraUniforms, CompositorUniforms, GaussianSceneSoa, GpuPipelineState,
+                           _abi, random_scene)
 from helpers import assert_stage23_exact, compositor, config0_camera, gpu_buffers, oracle_frame
 
 pytestmark = pytest.mark.gpu
@@ -189,5 +190,44 @@ def test_more_entries_than_a_frame_may_have():
         far = look(60.0, 320, 180)  # the context goes on
         small = compositor(320, 180, far, deg=0)
         assert st.execute_frame_gpu(scene, None, far, small, force_stage3=True).total_tile_entries > 0
+    finally:
+        st.close()
+
+
+@pytest.mark.parametrize("sort", [_abi.SORT_RADIX, _abi.SORT_TRANSPOSE, _abi.SORT_AUTO])
+def test_graph_of_views_of_different_widths(sort):
+    """The pass before a capture may raise the capacities without a re-render
+    (entries past 80% of them): the buffers then fit every view's digit width
+    when the graph is captured, and its replay equals the views one by one."""
+    w, h = 1920, 1080
+    scene = random_scene(4000, seed=13)
+    scene.covariances_3d[:] = np.array([0.09, 0.0, 0.0, 0.09, 0.0, 0.09], np.float32)
+    scene.positions *= np.float32(0.4)
+    cam = config0_camera(w, h)
+    st = GpuPipelineState(0)
+    st.upload_scene(scene)
+    all_entries = st.execute_frame_gpu(scene, None, cam, compositor(w, h, cam)).total_tile_entries
+    st.close()
+    n = int(scene.count * 0.92 * 2**20 / all_entries)
+    part = GaussianSceneSoa(scene.positions[:n], scene.covariances_3d[:n], scene.opacities[:n],
+                            scene.sh_coeffs[:n])
+    sizes = [(w, h), (640, 360), (64, 48)]  # 13, 10 and 4 tile bits
+    cams = [config0_camera(*s) for s in sizes]
+    comps = [compositor(*s, c, deg=1) for s, c in zip(sizes, cams)]
+    st = GpuPipelineState(0)
+    try:
+        st.upload_scene(part)
+        st.upload_cages(None)
+        images = st.view_images(comps)
+        stats = [st.execute_views(part, None, cams, comps, images, entry_sort=sort) for _ in range(3)]
+        assert stats[0]["views_rerendered"] == 0 or sort == _abi.SORT_AUTO
+        assert stats[-1]["graph_replayed"] == 1
+        torch.cuda.synchronize()
+        got = [im.cpu().numpy().view(np.uint8).reshape(s[1], s[0], 4) for im, s in zip(images, sizes)]
+        for s, c, q, im in zip(sizes, cams, comps, got):
+            t = st.execute_frame_gpu(part, None, c, q, force_stage3=True)
+            np.testing.assert_array_equal(im, st.readback_framebuffer_rgba8(*s))
+            if s == (w, h):
+                assert 0.8 * 2**20 < t.total_tile_entries <= 2**20
     finally:
         st.close()
